@@ -179,6 +179,17 @@ __device__ __forceinline__ void contribution(const Cx<R> *l, const Cx<R> *r, con
     }
 }
 
+// ops 7 and 8: the momentum's Weyl matrix applied to c
+template <int OP, class R> __device__ __forceinline__ void weyl_slash(const Cx<R> *c, const R *p, Cx<R> *o) {
+    if (OP == 7) {
+        o[0] = ((-times_i(scaled(c[0], p[3])) - times_i(scaled(c[1], p[1]))) + scaled(c[1], p[2])) + times_i(scaled(c[0], p[0]));
+        o[1] = ((-scaled(c[0], p[2]) - times_i(scaled(c[0], p[1]))) + times_i(scaled(c[1], p[0]))) + times_i(scaled(c[1], p[3]));
+    } else {
+        o[0] = ((-scaled(c[1], p[2]) + times_i(scaled(c[0], p[0]))) + times_i(scaled(c[0], p[3]))) + times_i(scaled(c[1], p[1]));
+        o[1] = ((-times_i(scaled(c[1], p[3])) + scaled(c[0], p[2])) + times_i(scaled(c[0], p[1]))) + times_i(scaled(c[1], p[0]));
+    }
+}
+
 // ops 7-9: the propagator applied to c (2 or 4 components) into o
 template <int OP, class R>
 __device__ __forceinline__ void propagator(const Cx<R> *c, const R *p, R reciprocal, Cx<R> f, Cx<R> *o) {
@@ -188,16 +199,10 @@ __device__ __forceinline__ void propagator(const Cx<R> *c, const R *p, R recipro
         for (int k = 0; k < 4; k++) o[k] = c[k] * s;
         return;
     }
-    Cx<R> s = scaled(f, reciprocal), a, b;
-    if (OP == 7) {
-        a = ((-times_i(scaled(c[0], p[3])) - times_i(scaled(c[1], p[1]))) + scaled(c[1], p[2])) + times_i(scaled(c[0], p[0]));
-        b = ((-scaled(c[0], p[2]) - times_i(scaled(c[0], p[1]))) + times_i(scaled(c[1], p[0]))) + times_i(scaled(c[1], p[3]));
-    } else {
-        a = ((-scaled(c[1], p[2]) + times_i(scaled(c[0], p[0]))) + times_i(scaled(c[0], p[3]))) + times_i(scaled(c[1], p[1]));
-        b = ((-times_i(scaled(c[1], p[3])) + scaled(c[0], p[2])) + times_i(scaled(c[0], p[1]))) + times_i(scaled(c[1], p[0]));
-    }
-    o[0] = a * s;
-    o[1] = b * s;
+    Cx<R> s = scaled(f, reciprocal), a[2];
+    weyl_slash<OP>(c, p, a);
+    o[0] = a[0] * s;
+    o[1] = a[1] * s;
 }
 
 // op 10: factor x value

@@ -82,13 +82,11 @@ struct pacuda_b200_batch {
 
 namespace {
 
-void fill_plan(const pacuda_b200_plan *p, TiledPlan &d, uint32_t points, int blocks = 1) {
+void fill_plan(const pacuda_b200_plan *p, TiledPlan &d, uint32_t points, size_t const_bytes, int blocks = 1) {
     memset(&d, 0, sizeof d);
-    describe(p->tiled, p->forms, points, p->point_bytes, d, blocks);
+    describe(p->tiled, p->forms, points, p->point_bytes, const_bytes, d, blocks);
     d.s64 = p->consts;
     d.f64 = p->consts + 2 * p->scales;
-    d.kconst = p->consts + 2 * (p->scales + p->factors);
-    d.scales = p->scales;
     d.factors = p->factors;
     d.form_terms = p->terms;
     d.term_slots = p->terms + 2 * p->forms;
@@ -116,7 +114,20 @@ Offsets layout(size_t n) {
 
 // blocks per SM chosen without timing (tiled_auto_blocks)
 int auto_blocks(const pacuda_b200_plan *p) {
-    return tiled_auto_blocks(p->kernel, p->point_bytes, tiled_const_bytes(p->scales, p->factors));
+    return tiled_auto_blocks(p->kernel, p->point_bytes, tiled_const_bytes(p->tiled));
+}
+
+// The shared memory that the blocks of a launch keep for its plans' folded entries: the largest
+// table, or none (the entries are then read from global memory) where a plan's point would not fit
+// beside it. `which`: the launch's plans among `plans` (null: the first n).
+size_t group_const_bytes(pacuda_b200_plan *const *plans, const uint32_t *which, size_t n, int kernel, int blocks) {
+    size_t table = 0, point = 0;
+    for (size_t j = 0; j < n; j++) {
+        const pacuda_b200_plan *p = plans[which ? which[j] : j];
+        table = std::max(table, tiled_const_bytes(p->tiled));
+        point = std::max(point, p->point_bytes);
+    }
+    return table + point <= tiled_max_smem(kernel, blocks) ? table : 0;
 }
 
 // The groups and the host block from the batch's current choices: each group's shared memory and
@@ -160,15 +171,8 @@ bool prepare(pacuda_b200_batch *b) {
         TiledPlan *plans = (TiledPlan *)(base + o.plans);
         unsigned long long *items = (unsigned long long *)(base + o.items);
         g.threads = tiled_threads(kernel, g.blocks);
-        g.const_bytes = 0;
-        for (uint32_t k : g.plans)
-            g.const_bytes = std::max(g.const_bytes, tiled_const_bytes(b->plans[k]->scales, b->plans[k]->factors));
-        size_t room = tiled_max_smem(kernel, g.blocks);
-        if (room <= g.const_bytes) {
-            fprintf(stderr, "%s: the plans' constants do not fit a block's shared memory\n", kTag);
-            return false;
-        }
-        size_t max_smem = room - g.const_bytes;
+        g.const_bytes = group_const_bytes(b->plans.data(), g.plans.data(), m, kernel, g.blocks);
+        const size_t max_smem = tiled_max_smem(kernel, g.blocks) - g.const_bytes;
         g.smem = 0;
         items[0] = 0;
         for (size_t j = 0; j < m; j++) {
@@ -184,7 +188,7 @@ bool prepare(pacuda_b200_batch *b) {
                                ? p->points
                                : tiled_default_points(p->point_bytes, g.threads, max_smem);
             b->points[k] = per;
-            fill_plan(p, plans[j], per, g.blocks);
+            fill_plan(p, plans[j], per, g.const_bytes, g.blocks);
             g.smem = std::max<size_t>(g.smem, (size_t)per * p->point_bytes);
             items[j + 1] = items[j] + (b->count[k] + per - 1) / per;
             ((const double **)(base + o.external))[j] = b->external[k];
@@ -231,7 +235,8 @@ int launch(pacuda_b200_batch *b, cudaStream_t s) {
 
 // the shared memory a block has for one plan's points
 size_t point_smem(const pacuda_b200_plan *p) {
-    return tiled_max_smem(p->kernel) - tiled_const_bytes(p->scales, p->factors);
+    pacuda_b200_plan *one = const_cast<pacuda_b200_plan *>(p);
+    return tiled_max_smem(p->kernel) - group_const_bytes(&one, nullptr, 1, p->kernel, 1);
 }
 
 // the default points per block (tiled_default_points)
@@ -319,14 +324,15 @@ extern "C" pacuda_b200_plan *pacuda_b200_plan_create(const pacman_recurrence_cal
               to_device(&p->coefficients, c->term_coefficients, c->term_count) &&
               to_device(&p->red_offsets, offsets, (size_t)outputs + 1) &&
               to_device(&p->red_slots, slots.data(), slots.size()) &&
-              to_device(&p->red_weights, weights, offsets[outputs]) && upload_schedule(p->tiled, tiled_threads(p->kernel), 0) &&
+              to_device(&p->red_weights, weights, offsets[outputs]) && upload_schedule(p->tiled, forms, p->kernel, tiled_threads(p->kernel), {c->scale_re, c->scale_im, c->factor_re, c->factor_im}, 0) &&
+              fold_values(p->tiled, p->kernel, p->consts + nc, p->scales, p->factors, 0) &&
               !failed(cudaDeviceSynchronize(), "plan upload");
     if (!ok) {
         if (!p->tiled.host.why.empty()) fprintf(stderr, "%s: plan_create: %s\n", kTag, p->tiled.host.why.c_str());
         pacuda_b200_plan_destroy(p);
         return nullptr;
     }
-    p->point_bytes = tiled_point_bytes(p->tiled.host, forms, p->kernel);
+    p->point_bytes = tiled_point_bytes(p->tiled, forms, p->kernel);
     p->points = default_points(p);
     return p;
 }
@@ -490,7 +496,7 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
     const int kernel = b->plans[0]->kernel;
     for (size_t k = 0; k < b->plans.size(); k++) {
         pacuda_b200_plan *p = b->plans[k];
-        size_t cb = tiled_const_bytes(p->scales, p->factors);
+        size_t cb = tiled_const_bytes(p->tiled);
         float best = -1.0f;
         uint32_t best_points = p->points;
         int best_blocks = 0;
@@ -724,18 +730,11 @@ extern "C" int pacuda_b200_run_static(pacuda_b200_plan *const *plans, uint32_t n
     // the launch's shape as a batch of these plans has it; the plans' own choices are not changed
     int kernel = plans[0]->kernel;
     int threads = tiled_threads(kernel);
-    size_t const_bytes = 0;
-    for (uint32_t k = 0; k < nplans; k++)
-        const_bytes = std::max(const_bytes, tiled_const_bytes(plans[k]->scales, plans[k]->factors));
     // the shared memory a block may have, less the plan constants every block holds (checked
     // before anything is queued)
     const size_t room = tiled_max_smem(kernel);
     if (room == 0) return PACMAN_RECURRENCE_DEVICE_ERROR;
-    if (room <= const_bytes) {
-        fprintf(stderr, "%s: run_static: the plans' constants (%zu bytes) fill a block's shared memory\n", kTag,
-                const_bytes);
-        return PACMAN_RECURRENCE_INVALID;
-    }
+    const size_t const_bytes = group_const_bytes(plans, nullptr, nplans, kernel, 1);
     const size_t max_smem = room - const_bytes;
     StaticBlock block;
     memset(&block, 0, sizeof block);
@@ -750,7 +749,7 @@ extern "C" int pacuda_b200_run_static(pacuda_b200_plan *const *plans, uint32_t n
         uint32_t per = tiled_points_fit(p->points, p->point_bytes, threads, max_smem)
                            ? p->points
                            : tiled_default_points(p->point_bytes, threads, max_smem);
-        fill_plan(p, block.plans[k], per);
+        fill_plan(p, block.plans[k], per, const_bytes);
         smem = std::max<size_t>(smem, (size_t)per * p->point_bytes);
         block.items[k + 1] = block.items[k] + (count[k] + per - 1) / per;
         block.external[k] = external[k];

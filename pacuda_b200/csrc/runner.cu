@@ -373,15 +373,16 @@ int onchip_launch(DeviceProgram *prog, const pacman_recurrence_call *c, const Ru
     if (prog->tiled_state == 0) {
         prog->tiled_state = -1;
         if (build_schedule(prog->host, c->current_planes, c->amplitude_planes, prog->tiled.host) &&
-            upload_schedule(prog->tiled, tiled_threads(kernel), dev.stream))
+            upload_schedule(prog->tiled, forms, kernel, tiled_threads(kernel), TiledConstants(), dev.stream))
             prog->tiled_state = 1;
     }
     // the lanes per point: as configured, else the default points per block; one block per SM (the
     // arena write-back of a block's interleaved points is coalesced over them: several blocks of
     // fewer points measured 19 % slower for gg>ggg through this path)
     int threads = prog->tiled_state == 1 ? tiled_threads(kernel) : 0;
-    size_t pb = prog->tiled_state == 1 ? tiled_point_bytes(prog->tiled.host, forms, kernel) : 0;
-    size_t cb = tiled_const_bytes(c->scale_count, c->factor_count);
+    size_t pb = prog->tiled_state == 1 ? tiled_point_bytes(prog->tiled, forms, kernel) : 0;
+    size_t cb = tiled_const_bytes(prog->tiled);
+    if (cb + pb > (threads ? tiled_max_smem(kernel) : 0)) cb = 0;  // (the entries stay in global memory)
     size_t room = threads ? tiled_max_smem(kernel) - cb : 0;
     uint32_t np = threads && prog->tiled.threads == threads ? tiled_default_points(pb, threads, room) : 0;
     if (np && current.lanes_per_point) {
@@ -399,12 +400,13 @@ int onchip_launch(DeviceProgram *prog, const pacman_recurrence_call *c, const Ru
     if (!dev.launch_dev.reserve(total, "descriptors")) return -1;
     memset(dev.launch_host, 0, total);
     TiledPlan &p = *(TiledPlan *)dev.launch_host;
-    describe(prog->tiled, forms, np, pb, p);
+    describe(prog->tiled, forms, np, pb, cb, p);
     p.s64 = a.s64;
     p.f64 = a.f64;
+    p.factors = a.factors;
+    p.entry_list = prog->tiled.entries;
     p.kconst = a.kconst;
     p.scales = a.scales;
-    p.factors = a.factors;
     p.form_terms = a.form_terms;
     p.term_slots = a.term_slots;
     p.coefficients = a.coefficients;
@@ -434,7 +436,9 @@ int onchip_launch(DeviceProgram *prog, const pacman_recurrence_call *c, const Ru
     L.mom = forms_on_device ? nullptr : a.mom;
     L.ld = a.ld;
     L.const_bytes = (uint32_t)cb;
-    if (!launch_tiled(kernel, L, threads, smem, dev.sms, dev.stream) || failed(cudaGetLastError(), "launch")) return -1;
+    // (a table that stays in global memory is folded here, for this call's constants)
+    if ((!cb && !fold_values(prog->tiled, kernel, a.kconst, a.scales, a.factors, dev.stream)) ||
+        !launch_tiled(kernel, L, threads, smem, dev.sms, dev.stream) || failed(cudaGetLastError(), "launch")) return -1;
     // the host descriptors are read by the copy: wait for it before a later call rewrites them
     return failed(cudaStreamSynchronize(dev.stream), "descriptors") ? -1 : 1;
 }

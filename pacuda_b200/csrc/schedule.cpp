@@ -2,9 +2,12 @@
 #include "schedule.h"
 
 #include <algorithm>
+#include <array>
+#include <cmath>
 #include <map>
 #include <numeric>
 #include <queue>
+#include <unordered_map>
 
 namespace pacuda {
 namespace {
@@ -531,6 +534,111 @@ bool use_terms(Schedule &s, const uint32_t *offsets, const uint32_t *planes, uin
     s.amp_slots = 0;
     s.amp_planes.clear();
     return true;
+}
+
+void fold_constants(const Schedule &s, const double *scale_re, const double *scale_im, const double *factor_re,
+                    const double *factor_im, Folds &out) {
+    out = Folds();
+    auto set_class = [](Ins &i, uint32_t c) { i.head = (i.head & 0xffff) | c << 16; };
+    const bool known = scale_re && scale_im && factor_re && factor_im;
+    std::unordered_map<uint64_t, uint32_t> entry_of, reciprocal_of;
+    std::map<std::array<uint32_t, 3>, uint32_t> run_of;  // closures' (first component, factor, count) -> first entry
+    auto entry = [&](uint32_t kind, uint32_t a, uint32_t b) {
+        auto it = entry_of.emplace((uint64_t)(kind << 28 | a) << 32 | b, (uint32_t)out.entries.size() / 2);
+        if (it.second) {
+            out.entries.push_back(kind << 28 | a);
+            out.entries.push_back(b);
+        }
+        return it.first->second;
+    };
+    out.ins.reserve(s.ins.size());
+    out.task_first.reserve(s.task_first.size());
+    // the class of (ar + i ai)(br + i bi): both products of its real (imaginary) part have an
+    // operand that is exactly zero, in f64 and so in every kind's rounding of it
+    auto class_of = [](double ar, double ai, double br, double bi) -> uint32_t {
+        if (!std::isfinite(ar) || !std::isfinite(ai) || !std::isfinite(br) || !std::isfinite(bi)) return C_GENERAL;
+        const bool real = (ar == 0.0 || bi == 0.0) && (ai == 0.0 || br == 0.0);
+        const bool imag = (ar == 0.0 || br == 0.0) && (ai == 0.0 || bi == 0.0);
+        if (real && ((ar == 1.0 && br == 1.0 && ai == 0.0 && bi == 0.0) || (ar == -1.0 && br == -1.0 && ai == 0.0 && bi == 0.0)))
+            return C_ONE;
+        return real ? C_REAL : imag ? C_IMAG : C_GENERAL;
+    };
+    for (size_t n = 0, task = 0; n < s.ins.size(); n++) {
+        while (task < s.task_first.size() && s.task_first[task] == n) {
+            out.task_first.push_back((uint32_t)out.ins.size());
+            task++;
+        }
+        Ins i = s.ins[n];
+        switch (ins_kind(i)) {
+        case K_CONTRIB: {
+            if ((ins_flags(i) & F_FIRST) && !(ins_flags(i) & F_INIT)) {
+                int c0, c1, cd;
+                contribution_shape(ins_op(i), &c0, &c1, &cd);
+                Ins load{};
+                load.head = K_CONTRIB | kOpLoad << 4;
+                load.c = i.c;
+                load.s = (uint32_t)cd;
+                set_class(load, C_GENERAL);
+                out.ins.push_back(load);
+            }
+            const uint32_t scale = i.s, factor = i.x;
+            i.s = entry(FOLD_SCALE_FACTOR, scale, factor);
+            set_class(i, known ? class_of(scale_re[scale], scale_im[scale], factor_re[factor], factor_im[factor]) : C_GENERAL);
+            break;
+        }
+        case K_PROP: {
+            const uint32_t factor = i.x, op = ins_op(i);
+            auto r = reciprocal_of.emplace(i.f, (uint32_t)out.reciprocals.size());
+            if (r.second) out.reciprocals.push_back(i.f);
+            i.s = r.first->second;
+            i.x = op == 9 ? entry(FOLD_MINUS_I, factor, 0) : entry(FOLD_FACTOR, factor, 0);
+            set_class(i, !known ? C_GENERAL
+                                : op == 9 ? class_of(factor_re[factor], factor_im[factor], 0.0, -1.0)
+                                          : class_of(factor_re[factor], factor_im[factor], 1.0, 0.0));
+            break;
+        }
+        case K_IDENTITY: i.x = entry(FOLD_FACTOR, i.x, 0); break;
+        case K_CLOSURE: {
+            // the components' entries stand next to each other (closures of one pattern share them)
+            const uint32_t first = i.y, factor = i.x;
+            auto r = run_of.emplace(std::array<uint32_t, 3>{first, factor, i.s}, (uint32_t)out.entries.size() / 2);
+            if (r.second)
+                for (uint32_t k = 0; k < i.s; k++) {
+                    out.entries.push_back(FOLD_FACTOR_FACTOR << 28 | (first + k));
+                    out.entries.push_back(factor);
+                }
+            i.y = r.first->second;
+            uint32_t cls = known ? C_REAL : C_GENERAL;
+            for (uint32_t k = 0; known && k < i.s; k++) {
+                const uint32_t c = class_of(factor_re[first + k], factor_im[first + k], factor_re[factor], factor_im[factor]);
+                if (c != C_REAL && c != C_ONE) cls = C_GENERAL;
+            }
+            i.x = 0;
+            set_class(i, cls);
+            break;
+        }
+        default: break;  // clears have no constants; sources read theirs in f64
+        }
+        out.ins.push_back(i);
+    }
+    out.task_first.resize(s.task_first.size(), (uint32_t)out.ins.size());  // (the end of the last task)
+}
+
+uint32_t row_code(const Ins &i) {
+    const uint32_t op = ins_op(i), cls = ins_count(i), flags = ins_flags(i);
+    if (ins_kind(i) == K_CONTRIB && op != kOpLoad) {
+        if (op == 4 && cls == C_IMAG) return R_TENSOR_IMAG;
+        if (op == 6 && cls == C_IMAG) return R_VECTOR_IMAG;
+        if (op == 5 && cls == C_ONE) return R_WEDGE_ONE;
+        if (op == 2 && cls == C_REAL) return R_WEYL_A_REAL;
+        if (op == 3 && cls == C_REAL) return R_WEYL_B_REAL;
+    }
+    if (ins_kind(i) == K_PROP && op == 9 && cls == C_IMAG && i.s != kNoReciprocal) return R_PROP_IMAG;
+    if (ins_kind(i) == K_CLOSURE && cls == C_REAL && (flags & F_ACC0) && (flags & F_TERM) && i.c != 0xffff) {
+        if (i.s == 4) return R_CLOSE4_REAL;
+        if (i.s == 2) return R_CLOSE2_REAL;
+    }
+    return R_OTHER;
 }
 
 }  // namespace pacuda

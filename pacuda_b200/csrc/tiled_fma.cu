@@ -14,4 +14,10 @@ const void *tiled_fma_kernel(bool abi) {
     return abi ? (const void *)run_tiled<KindF64Fma, true> : (const void *)run_tiled<KindF64Fma, false>;
 }
 
+void tiled_fma_fold(const uint32_t *entries, uint32_t count, const void *constants, uint32_t scales, uint32_t factors,
+                    void *out, cudaStream_t s) {
+    fold_constants_kernel<KindF64Fma><<<(count + 127) / 128, 128, 0, s>>>(entries, count, (const double *)constants,
+                                                                          scales, factors, (Pair<double> *)out);
+}
+
 }  // namespace pacuda

@@ -21,6 +21,8 @@ template <class T> bool put(T **dst, const std::vector<T> &v, cudaStream_t s) {
 
 // the f64 kind with contracted multiply-adds (tiled_fma.cu, compiled with -fmad=true)
 const void *tiled_fma_kernel(bool abi);
+void tiled_fma_fold(const uint32_t *entries, uint32_t count, const void *constants, uint32_t scales, uint32_t factors,
+                    void *out, cudaStream_t s);
 
 namespace {
 
@@ -41,43 +43,71 @@ const void *kernel_for(int kernel, bool abi = false) {
 
 void TiledDevice::release() {
     cudaFree(ins);
-    cudaFree(task_first);
     cudaFree(loads);
     cudaFree(amp_planes);
     cudaFree(orders);
     cudaFree(level_firsts);
+    cudaFree(entries);
+    cudaFree(recip_forms);
+    cudaFree(folded);
     ins = nullptr;
-    task_first = loads = amp_planes = orders = level_firsts = nullptr;
+    loads = amp_planes = orders = level_firsts = entries = recip_forms = nullptr;
+    folded = nullptr;
     ok = false;
 }
 
-bool pack_ins(const Ins &i, uint4 &w) {
+bool pack_ins(const Ins &i, bool end, uint4 &w) {
     // (a closure's f records its global amplitude plane for the host; the executor reads its slot)
     uint32_t f = ins_kind(i) == K_CLOSURE ? 0 : i.f, f0 = f & 0xffff, f1 = f >> 16;
-    if (ins_flags(i) > 255 || f0 > 255 || f1 > 255 || i.a > 0xffff || i.b > 0xffff || i.c > 0xffff || i.s > 0xffff ||
+    if (ins_count(i) > C_GENERAL || f0 > 255 || f1 > 255 || i.a > 0xffff || i.b > 0xffff || i.c > 0xffff || i.s > 0xffff ||
         i.x > 0xffff || i.y > 0xffff)
         return false;
-    w.x = (i.head & 0xffff) | f0 << 16 | f1 << 24;
+    const uint32_t flags = ins_flags(i);
+    const bool contribution = ins_kind(i) == K_CONTRIB && ins_op(i) != kOpLoad, last = !contribution || (flags & F_LAST);
+    uint32_t head = row_code(i) | ins_count(i) << 4 | ins_op(i) << 8;
+    if (end) head |= H_END;
+    if (contribution && last && !(flags & F_NOSTORE)) head |= H_STORE;
+    if (flags & F_ACC0) head |= H_ACC0;
+    if (flags & F_TERM) head |= H_TERM;
+    if (contribution && (flags & F_FIRST) && (flags & F_INIT)) head |= H_SET;
+    if (last && (flags & F_WB)) head |= H_WB;
+    w.x = head | f0 << 16 | f1 << 24;
     w.y = i.a | i.b << 16;
     w.z = i.c | i.s << 16;
     w.w = i.x | i.y << 16;
     return true;
 }
 
-bool upload_schedule(TiledDevice &t, int threads, cudaStream_t s) {
-    std::vector<uint4> packed(t.host.ins.size());
+bool upload_schedule(TiledDevice &t, uint32_t forms, int kernel, int threads, const TiledConstants &c, cudaStream_t s) {
+    Folds folds;
+    fold_constants(t.host, c.scale_re, c.scale_im, c.factor_re, c.factor_im, folds);
+    t.entry_count = (uint32_t)folds.entries.size() / 2;
+    t.recips = (uint32_t)folds.reciprocals.size();
+    if (tiled_const_bytes(t) + tiled_point_bytes(t, forms, kernel) > tiled_max_smem(kernel)) {
+        // (a point at the limit of the shared memory: its propagators keep computing theirs)
+        t.recips = 0;
+        folds.reciprocals.clear();
+        for (Ins &i : folds.ins)
+            if (ins_kind(i) == K_PROP) i.s = kNoReciprocal;
+    }
+    std::vector<uint8_t> end(folds.ins.size(), 0);
+    for (size_t k = 1; k < folds.task_first.size(); k++) end[folds.task_first[k] - 1] = 1;
+    std::vector<uint4> packed(folds.ins.size());
     for (size_t n = 0; n < packed.size(); n++)
-        if (!pack_ins(t.host.ins[n], packed[n])) {
+        if (!pack_ins(folds.ins[n], end[n], packed[n])) {
             t.host.why = "an instruction's field does not fit the on-chip executor's 16-byte form";
             t.ok = false;
             return false;
         }
-    packed.push_back(make_uint4(0, 0, 0, 0));  // read (not run) by the prefetch after a task's last row
-    t.ok = threads > 0 && put(&t.ins, packed, s) && put(&t.task_first, t.host.task_first, s) &&
-           put(&t.loads, t.host.loads, s) && put(&t.amp_planes, t.host.amp_planes, s);
+    // fetched (not run) ahead of a task's end, and beside the positions without a task
+    const uint32_t padding = (uint32_t)packed.size();
+    packed.resize(packed.size() + 8, make_uint4(0, 0, 0, 0));
+    t.ok = threads > 0 && put(&t.ins, packed, s) && put(&t.loads, t.host.loads, s) && put(&t.amp_planes, t.host.amp_planes, s) &&
+           put(&t.entries, folds.entries, s) && put(&t.recip_forms, folds.reciprocals, s) &&
+           cudaMalloc(&t.folded, std::max<size_t>(1, t.entry_count) * 16) == cudaSuccess;
     t.levels = (uint32_t)t.host.level_first.size() - 1;
     t.threads = threads;
-    std::vector<uint32_t> ranges, firsts;
+    std::vector<uint32_t> first, firsts;
     // one order per distinct lane count: blocks of b per SM with P points give
     // tiled_lanes(P, tiled_block_threads(threads, b)) lanes, and many pairs give the same count
     std::vector<bool> made(kMaxLanes + 1, false);
@@ -88,29 +118,42 @@ bool upload_schedule(TiledDevice &t, int threads, cudaStream_t s) {
             made[lanes] = true;
             std::vector<uint32_t> order, lf;
             lane_order(t.host, lanes, order, lf);
-            // each position holds its task's instruction range (first, end); (0, 0) for none
-            t.order_at[lanes] = ranges.size();
+            // each position holds its task's first instruction
+            t.order_at[lanes] = first.size();
             t.level_at[lanes] = firsts.size();
-            for (uint32_t task : order) {
-                ranges.push_back(task == ~0u ? 0 : t.host.task_first[task]);
-                ranges.push_back(task == ~0u ? 0 : t.host.task_first[task + 1]);
-            }
+            for (uint32_t task : order) first.push_back(task == ~0u ? kNoTask | padding : folds.task_first[task]);
             firsts.insert(firsts.end(), lf.begin(), lf.end());
         }
-    // the executor fetches the next position of a lane before testing it against the level's end:
-    // up to a lane count past the last one
-    ranges.insert(ranges.end(), 2 * kMaxLanes, 0);
-    t.ok = t.ok && put(&t.orders, ranges, s) && put(&t.level_firsts, firsts, s);
+    // the executor fetches two positions of a lane ahead: up to two lane counts past the last one
+    first.insert(first.end(), 3 * kMaxLanes, kNoTask | padding);
+    t.ok = t.ok && put(&t.orders, first, s) && put(&t.level_firsts, firsts, s);
     // the host vectors must outlive the asynchronous copies
     cudaStreamSynchronize(s);
     return t.ok;
 }
 
-size_t tiled_const_bytes(uint32_t scales, uint32_t factors) { return ((2 * (size_t)scales + 2 * factors) * 8 + 15) / 16 * 16; }
+bool fold_values(const TiledDevice &t, int kernel, const void *constants, uint32_t scales, uint32_t factors,
+                 cudaStream_t s) {
+    if (!t.entry_count) return true;
+    auto fold = [&](auto k) {
+        typedef decltype(k) K;
+        fold_constants_kernel<K><<<(t.entry_count + 127) / 128, 128, 0, s>>>(
+            t.entries, t.entry_count, (const typename K::Const *)constants, scales, factors, (Pair<typename K::R> *)t.folded);
+    };
+    switch (kernel) {
+    case PACMAN_RECURRENCE_KERNEL_F64: fold(KindF64()); break;
+    case PACUDA_B200_KERNEL_F64_FMA: tiled_fma_fold(t.entries, t.entry_count, constants, scales, factors, t.folded, s); break;
+    case PACMAN_RECURRENCE_KERNEL_MIXED: fold(KindMixed()); break;
+    case PACMAN_RECURRENCE_KERNEL_MIXED64: fold(KindMixed64()); break;
+    default: fold(KindDF64()); break;
+    }
+    return cudaGetLastError() == cudaSuccess;
+}
 
-size_t tiled_point_bytes(const Schedule &s, uint32_t forms, int kernel) {
+size_t tiled_point_bytes(const TiledDevice &t, uint32_t forms, int kernel) {
+    const Schedule &s = t.host;
     size_t value = kernel == PACMAN_RECURRENCE_KERNEL_MIXED || kernel == PACMAN_RECURRENCE_KERNEL_MIXED64 ? 4 : 8;
-    size_t per_point = 2 * value * s.cur_slots + 2 * 8 * s.amp_slots + 8 * (size_t)s.terms + 8 * 4 * (size_t)forms;
+    size_t per_point = 2 * value * s.cur_slots + 2 * 8 * s.amp_slots + 8 * ((size_t)s.terms + t.recips) + 8 * 4 * (size_t)forms;
     return (per_point + 15) / 16 * 16;
 }
 
@@ -180,9 +223,9 @@ uint32_t tiled_default_points(size_t point_bytes, int threads, size_t max_smem) 
     return best;
 }
 
-void describe(const TiledDevice &t, uint32_t forms, uint32_t points, size_t point_bytes, TiledPlan &p, int blocks) {
+void describe(const TiledDevice &t, uint32_t forms, uint32_t points, size_t point_bytes, size_t const_bytes, TiledPlan &p,
+              int blocks) {
     p.ins = t.ins;
-    p.task_first = t.task_first;
     const uint32_t lanes = tiled_lanes(points, tiled_block_threads(t.threads, blocks));
     p.order = t.orders + t.order_at[lanes];
     p.level_first = t.level_firsts + t.level_at[lanes];
@@ -197,6 +240,11 @@ void describe(const TiledDevice &t, uint32_t forms, uint32_t points, size_t poin
     p.loads = t.loads;
     p.nloads = (uint32_t)t.host.loads.size() / 3;
     p.amp_planes = t.amp_planes;
+    p.folded = t.folded;
+    p.entries = t.entry_count;
+    p.near = 16 * (size_t)t.entry_count <= const_bytes ? t.entry_count : 0;
+    p.recip_forms = t.recip_forms;
+    p.recips = t.recips;
 }
 
 bool launch_tiled(int kernel, const TiledLaunch &args, int threads, size_t smem, int grid, cudaStream_t stream) {

@@ -35,7 +35,11 @@ constexpr uint32_t kMaxLanes = 512;
 struct TiledDevice {
     Schedule host;
     uint4 *ins = nullptr;  // the schedule's instructions, packed (pack_ins)
-    uint32_t *task_first = nullptr, *loads = nullptr, *amp_planes = nullptr;
+    uint32_t *loads = nullptr, *amp_planes = nullptr;
+    // the folded constants' entries (schedule.h Folds) and values, the reciprocals' forms
+    uint32_t *entries = nullptr, *recip_forms = nullptr;
+    void *folded = nullptr;
+    uint32_t entry_count = 0, recips = 0;
     // per lane count G (of every blocks-per-SM choice and points per block): the lane order for G
     // lanes and its level boundaries, concatenated (offsets in 32-bit words, index G)
     uint32_t *orders = nullptr, *level_firsts = nullptr;
@@ -46,19 +50,30 @@ struct TiledDevice {
     void release();
 };
 
-// bytes of shared memory a block needs for one plan's constants (scales and factors, re and im)
-size_t tiled_const_bytes(uint32_t scales, uint32_t factors);
+// bytes of shared memory a block keeps for a plan's folded entries (0 for a large table, which is
+// read from global memory)
+constexpr uint32_t kNearEntries = 256;
+inline size_t tiled_const_bytes(const TiledDevice &t) { return t.entry_count <= kNearEntries ? 16 * (size_t)t.entry_count : 0; }
 
-// an instruction in the on-chip executor's 16-byte form (tiled.cuh unpack_ins); false when a field
-// does not fit it
-bool pack_ins(const Ins &i, uint4 &w);
+// a folded instruction (schedule.h Folds; `end`: its task's last) in the on-chip executor's 16-byte
+// form (tiled.cuh Row16); false when a field does not fit it
+bool pack_ins(const Ins &i, bool end, uint4 &w);
 
+// the constants that a plan's classes are read from (null pointers: none known, every class general)
+struct TiledConstants {
+    const double *scale_re = nullptr, *scale_im = nullptr, *factor_re = nullptr, *factor_im = nullptr;
+};
 // the schedule's arrays on the device, with the lane orders of every points-per-block count for
-// blocks of `threads`; false (with the reason in t.host.why) when an instruction does not pack
-bool upload_schedule(TiledDevice &t, int threads, cudaStream_t stream);
+// blocks of `threads` of kernel kind `kernel`; false (with the reason in t.host.why) when an
+// instruction does not pack. A point keeps its reciprocals where one point still fits a block with
+// them, else (none kept) each propagator computes its own.
+bool upload_schedule(TiledDevice &t, uint32_t forms, int kernel, int threads, const TiledConstants &c, cudaStream_t stream);
+// fills t.folded from the constants in the kind's layout (device: scales re, im, factors re, im)
+bool fold_values(const TiledDevice &t, int kernel, const void *constants, uint32_t scales, uint32_t factors,
+                 cudaStream_t stream);
 
 // bytes of shared memory one point needs (kernel: PACMAN_RECURRENCE_KERNEL_*), 16-aligned
-size_t tiled_point_bytes(const Schedule &s, uint32_t forms, int kernel);
+size_t tiled_point_bytes(const TiledDevice &t, uint32_t forms, int kernel);
 
 // a block's threads with `blocks` blocks per SM (as the kernel's registers allow, at most 512 per
 // SM) and its largest dynamic shared memory
@@ -82,7 +97,9 @@ int tiled_auto_blocks(int kernel, size_t point_bytes, size_t const_bytes);
 uint32_t tiled_default_points(size_t point_bytes, int threads, size_t max_smem);
 
 // fills the schedule fields of a plan descriptor for `points` points per block, `blocks` per SM
-void describe(const TiledDevice &t, uint32_t forms, uint32_t points, size_t point_bytes, TiledPlan &p, int blocks = 1);
+// with `const_bytes` of the block's shared memory for folded entries
+void describe(const TiledDevice &t, uint32_t forms, uint32_t points, size_t point_bytes, size_t const_bytes, TiledPlan &p,
+              int blocks = 1);
 
 // launches the persistent kernel (`grid` blocks: the SMs times the blocks per SM) with `smem` bytes
 // of shared memory

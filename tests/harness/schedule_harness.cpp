@@ -120,3 +120,31 @@ int schedule_export_terms(const uint64_t *words, uint32_t count, const uint8_t *
     return 0;
 }
 }
+
+extern "C" {
+// the folded constants of a plan's schedule: sizes = ins, entries, reciprocals; per instruction its 8
+// words and its dispatch code, the entries (2 words each), the reciprocals' forms
+int fold_export(const uint64_t *words, uint32_t count, const uint8_t *width, uint32_t planes, uint32_t amps,
+                uint32_t forms, uint32_t scales, uint32_t factors, const double *scale_re, const double *scale_im,
+                const double *factor_re, const double *factor_im, uint32_t *sizes, uint32_t *ins, uint32_t *codes,
+                uint32_t *entries, uint32_t *reciprocals) {
+    Program p;
+    Limits lim{planes, amps, forms, scales, factors};
+    BuildError e = build_program(words, count, width, true, lim, p);
+    if (e.status) return e.status;
+    Schedule s;
+    if (!build_schedule(p, planes, amps, s)) return -1;
+    Folds f;
+    fold_constants(s, scale_re, scale_im, factor_re, factor_im, f);
+    sizes[0] = (uint32_t)f.ins.size();
+    sizes[1] = (uint32_t)f.entries.size() / 2;
+    sizes[2] = (uint32_t)f.reciprocals.size();
+    if (ins) {
+        memcpy(ins, f.ins.data(), f.ins.size() * sizeof(Ins));
+        for (size_t n = 0; n < f.ins.size(); n++) codes[n] = row_code(f.ins[n]);
+        memcpy(entries, f.entries.data(), f.entries.size() * 4);
+        memcpy(reciprocals, f.reciprocals.data(), f.reciprocals.size() * 4);
+    }
+    return 0;
+}
+}
