@@ -157,9 +157,10 @@ int pacuda_uw_decide(uint64_t seed, const uint64_t *index, uint32_t n, uint32_t 
                      uint32_t helicities, const double *jac, const double *s, double w_max, double s_max,
                      double r_max, uint8_t *keep, double *weight, double *me, void *stream);
 
-/* Blocks per SM of the fused inference kernel (pacuda_sg_forward, the first stage): 2 (the
- * default; two blocks whose products and epilogues overlap, a 2-stage weight ring each) or 1 (one
- * block with a 9-stage weight ring); INVALID otherwise. Applies to later launches in the process. */
+/* Tiles of 128 points in flight per SM in the fused inference kernel (pacuda_sg_forward, the first
+ * stage): 2 (the default; one tile's products run behind the other's activations, where there are
+ * more tiles than SMs) or 1; INVALID otherwise. The outputs' bits do not depend on it. Applies to
+ * later launches in the process. */
 int pacuda_sg_set_inference_blocks(uint32_t blocks);
 
 /* kernel launches made by the last call of each entry point (0 for none) */

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(128, 1) gemm_kernel(GemmArgs g) {
     __shared__ float scal[4][2];
     const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
     uint8_t *smem = smem_raw + pad;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = (int)uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t mt = blockIdx.x, split = blockIdx.y;
     constexpr uint32_t COLS = N < 32 ? 32 : N;
 
@@ -195,23 +195,27 @@ __global__ void __launch_bounds__(128, 1) gemm_kernel(GemmArgs g) {
         // the copies still in flight end before the block does
         for (uint32_t i = issued > (uint32_t)S::STAGES ? issued - S::STAGES : 0; i < issued; i++)
             if (!mbar_wait(&full[i % S::STAGES], (i / S::STAGES) & 1, WAIT_CYCLES)) flag_error(g.error, 102, &abort_flag);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // the MMA issuer: 4 steps of K = 16 per tile
         constexpr uint32_t idesc = idesc_bf16(128, N);
-        for (uint32_t i = 0; i < g.k_tiles && !abort_flag; i++) {
+        const bool leader = elect_one();
+        for (uint32_t i = 0; i < g.k_tiles; i++) {
             const int s = i % S::STAGES;
-            if (!mbar_wait(&full[s], (i / S::STAGES) & 1, WAIT_CYCLES)) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (i / S::STAGES) & 1, WAIT_CYCLES))) {
                 flag_error(g.error, 103, &abort_flag);
                 break;
             }
             tc_fence_after();
-            const uint32_t a_addr = smem_u32(smem + (size_t)s * S::STAGE), b_addr = a_addr + S::A_BYTES;
+            const uint32_t a_addr = smem_u32(smem) + s * S::STAGE, b_addr = a_addr + S::A_BYTES;
+            if (leader) {
 #pragma unroll
-            for (uint32_t k = 0; k < 4; k++)
-                mma_bf16(tmem, sw128_desc(a_addr + 32 * k), sw128_desc(b_addr + 32 * k), idesc, (i | k) != 0);
-            mma_commit(&empty[s]);
+                for (uint32_t k = 0; k < 4; k++)
+                    mma_bf16(tmem, sw128_desc(a_addr + 32 * k), sw128_desc(b_addr + 32 * k), idesc, (i | k) != 0);
+                mma_commit(&empty[s]);
+            }
+            __syncwarp();
         }
-        mma_commit(&done);
+        if (leader) mma_commit(&done);
     }
     __syncwarp();
     // warp-uniform from here on: the tensor-memory loads below are .sync.aligned
@@ -454,25 +458,35 @@ __global__ void adam_kernel(float *params, float *m1, float *m2, const float *gr
 
 // ---- fused inference ------------------------------------------------------------------------------
 //
-// One block per 128 points at a time (persistent, two blocks per SM so that one block's products
-// run while the other's epilogue does): warps 0-7 build the inputs and run the epilogues (thread
-// (w, lane) owns point r = 32 (w % 4) + lane, tensor-memory lane r, and the column half w / 4),
-// warp 8 streams the weight images through a ring of two 16 KB stages (tiles of 128 rows x 64
-// values: chunk (k tile, half) of each layer), warp 9 issues the products (M = 128, N = 128 per
-// half) into 256 FP32 columns of tensor memory. The activations stay in one 64 KB A tile set,
-// overwritten in place by each epilogue once the layer's products have completed. The biases and
-// the output layer's weights sit in shared memory.
+// One persistent block per SM with two tiles of 128 points in flight. Warps 0-15 (eight per tile)
+// build the inputs and run the epilogues: thread (quarter, lane, c) owns point r = 32 quarter + lane,
+// tensor-memory lane r, and in each 128-column half of a layer the 64 columns of quarter c. Warp 16
+// streams the weight images through a ring of 16 KB chunks (half, k tile: 128 output rows x 64
+// values), each used by both tiles; warps 17 and 18 issue the tiles' products (M = 128, N = 128)
+// into 256 FP32 columns of tensor memory per tile. A tile's activations stay in one 64 KB A tile set.
+//
+// What bounds it is the activations: 1024 tanh per point on 16 MUFU lanes per SM are 64 cycles, the
+// products 52; so the products have to run behind the epilogues. A layer's products go half by half:
+// the first half's epilogue runs while the second half is computed (its results wait packed in 32
+// registers, since the products still read the activations they replace), and the next layer's
+// products start on the first half's k tiles while the second half's epilogue runs. Each tile has its
+// own issuing warp (one issues while the other waits), and the tiles' epilogues take turns, so that
+// one tile's activations run while the other's stores, barriers and products do; a warp loads its
+// accumulators before its turn. Sharing each chunk between two tiles halves the weights' L2 traffic.
+// Measured on B200, 2^21 points: 0.823 ms (109 cycles per point and SM, 1086 TFLOP/s, 0.65 of the
+// measured BF16 peak); 0.846 with the accumulators loaded inside the turns, 0.903 without turns, 1.25
+// with one issuing warp for both tiles, 1.44 with that warp's loop on one lane (umma.cuh elect_one).
+// The form before (two blocks per SM, a tile each, a layer's products and its epilogue one after the
+// other): 1.31 ms. 300 007 points: 192 -> 126 us.
+// Each output's sums keep their order (k tiles 0 .. 3; the output layer's 128 columns of a half one
+// after the other): the bits do not depend on the split.
 
-constexpr int FWD_EPI_THREADS = 256;
-constexpr int FWD_THREADS = FWD_EPI_THREADS + 64;
+constexpr int FWD_TILE_THREADS = 256;
+constexpr int FWD_THREADS = 2 * FWD_TILE_THREADS + 96;
 constexpr uint32_t FWD_CHUNK = 128 * 128;  // 16 KB
-// the weight ring's stages for one or two blocks per SM (the shared memory left beside the 64 KB of
-// activations), and the dynamic shared memory of a block
-template <int CTAS> struct FwdShape {
-    static constexpr int STAGES = CTAS == 1 ? 9 : 2;
-    static constexpr uint32_t SMEM = 4 * TILE_A + STAGES * FWD_CHUNK + 1024;
-};
-constexpr int FWD_CHUNKS = 2 + 3 * 8;  // per tile: layer 1 (1 k tile x 2 halves), layers 2-4 (4 x 2)
+constexpr int FWD_STAGES = 5;
+constexpr uint32_t FWD_SMEM = 8 * TILE_A + FWD_STAGES * FWD_CHUNK + 1024;
+constexpr int FWD_CHUNKS = 2 + 3 * 8;  // per tile: layer 1 (2 halves x 1 k tile), layers 2-4 (2 x 4)
 constexpr int FWD_PARAMS = 5 * WIDTH + 1;  // b1..b4, w5, b5
 
 struct ForwardArgs {
@@ -480,6 +494,7 @@ struct ForwardArgs {
     const float *params;
     const float *x;
     uint32_t inputs, count, tiles;
+    uint32_t per;  // tiles in flight per block: 2 or 1
     float *out;
     int *error;
     // candidates (stage 1 of two-stage unweighting): segments of candidates, one per subprocess;
@@ -501,42 +516,76 @@ __device__ __forceinline__ uint32_t segment_of(const ForwardArgs &g, uint32_t t)
 
 enum { FWD_FROM_X = 0, FWD_CANDIDATES = 1 };
 
-// chunk c of a tile's stream: its layer, k tile and half
-__device__ __forceinline__ void fwd_chunk(int c, int &layer, int &kt, int &half) {
-    if (c < 2) {
-        layer = 0;
-        kt = 0;
-        half = c;
-    } else {
-        layer = 1 + (c - 2) / 8;
-        kt = ((c - 2) % 8) / 2;
-        half = (c - 2) % 2;
-    }
+// the byte offset of chunk c of a tile's stream in the weight images (layer by layer, half by half,
+// its k tiles in order)
+__device__ __forceinline__ size_t fwd_chunk(uint32_t c) {
+    if (c < 2) return wimg_at(0) + (size_t)c * FWD_CHUNK;
+    const uint32_t layer = 1 + (c - 2) / 8, half = (c - 2) % 8 / 4, kt = (c - 2) % 4;
+    return wimg_at((int)layer) + (size_t)kt * 256 * 128 + (size_t)half * FWD_CHUNK;
 }
 
-template <int MODE, int CTAS>
-__global__ void __launch_bounds__(FWD_THREADS, CTAS) forward_kernel(ForwardArgs g) {
-    constexpr int FWD_STAGES = FwdShape<CTAS>::STAGES;
+// 64 columns of tensor memory from `taddr` (loaded while the warp waits for its turn)
+__device__ __forceinline__ void fwd_load(uint32_t taddr, uint32_t (&z)[4][16]) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) tmem_load16_async(taddr + 16 * k, z[k]);
+#pragma unroll
+    for (int k = 0; k < 4; k++) tmem_wait16(z[k]);
+}
+
+// four values through the activation, as two packed BF16 pairs; halved biases: the epilogue works on
+// z / 2 (in pairs: the single conversion shares the MUFU's pipe)
+__device__ __forceinline__ void fwd_activate4(const uint32_t *z, float4 b, uint32_t &lo, uint32_t &hi) {
+    lo = pack_bf16(silu_of_half(fmaf(__uint_as_float(z[0]), 0.5f, b.x)), silu_of_half(fmaf(__uint_as_float(z[1]), 0.5f, b.y)));
+    hi = pack_bf16(silu_of_half(fmaf(__uint_as_float(z[2]), 0.5f, b.z)), silu_of_half(fmaf(__uint_as_float(z[3]), 0.5f, b.w)));
+}
+
+__device__ __forceinline__ void fwd_activate(const uint32_t (&z)[4][16], const float *bias, uint32_t (&ph)[32]) {
+    const float4 *b4 = reinterpret_cast<const float4 *>(bias);
+#pragma unroll
+    for (int q = 0; q < 16; q++) fwd_activate4(&z[q / 4][4 * (q % 4)], b4[q], ph[2 * q], ph[2 * q + 1]);
+}
+
+// row r of one A tile from 32 packed pairs
+__device__ __forceinline__ void fwd_store_row(uint8_t *tile, uint32_t r, const uint32_t (&ph)[32]) {
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        *reinterpret_cast<uint4 *>(tile + sw128_offset(r, 8 * q)) =
+            make_uint4(ph[4 * q], ph[4 * q + 1], ph[4 * q + 2], ph[4 * q + 3]);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(FWD_THREADS, 1) forward_kernel(ForwardArgs g) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full[FWD_STAGES], empty[FWD_STAGES], act_ready, acc_ready, dot_ready;
+    __shared__ uint64_t full[FWD_STAGES], empty[FWD_STAGES];
+    // per tile: the activations' first and second 128 columns are written (the inputs are the first),
+    // a layer's first and second half of products is done, the output layer's second half is summed
+    __shared__ uint64_t act_ready[2][2], acc_ready[2][2], dot_ready[2];
+    __shared__ uint64_t turn[2];  // the other tile's warps have finished an epilogue
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
     __shared__ __align__(16) float prm[FWD_PARAMS];
-    __shared__ float dot_hi[128];
+    __shared__ float dot_hi[2][128];
     const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
-    uint8_t *act = smem_raw + pad;         // 4 A tiles: the activations (K = 256)
-    uint8_t *ring = act + 4 * TILE_A;      // weight chunks
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t my_tiles = blockIdx.x < g.tiles ? (g.tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    uint8_t *act = smem_raw + pad;         // per tile 4 A tiles: its activations (K = 256)
+    uint8_t *ring = act + 8 * TILE_A;      // weight chunks
+    const int warp = (int)uniform_warp(), lane = threadIdx.x & 31;
+    // the block's turns: turn i takes tiles per x (blockIdx + i gridDim) + 0 .. per - 1
+    const uint32_t pairs = (g.tiles + g.per - 1) / g.per;
+    const uint32_t turns = blockIdx.x < pairs ? (pairs - 1 - blockIdx.x) / gridDim.x + 1 : 0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < FWD_STAGES; s++) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
+            mbar_init(&empty[s], g.per);
         }
-        mbar_init(&act_ready, FWD_EPI_THREADS);
-        mbar_init(&acc_ready, 1);
-        mbar_init(&dot_ready, FWD_EPI_THREADS / 2);
+        for (int t = 0; t < 2; t++) {
+            for (int h = 0; h < 2; h++) {
+                mbar_init(&act_ready[t][h], FWD_TILE_THREADS);
+                mbar_init(&acc_ready[t][h], 1);
+            }
+            mbar_init(&dot_ready[t], FWD_TILE_THREADS / 2);
+            mbar_init(&turn[t], FWD_TILE_THREADS / 32);
+        }
         abort_flag = 0;
         fence_mbar_init();
     }
@@ -544,15 +593,15 @@ __global__ void __launch_bounds__(FWD_THREADS, CTAS) forward_kernel(ForwardArgs 
     // (P_W5, P_B5 follow each other)
     for (int i = threadIdx.x; i < FWD_PARAMS; i += FWD_THREADS)
         prm[i] = i < 4 * WIDTH ? 0.5f * g.params[bias_at(i / WIDTH) + i % WIDTH] : g.params[P_W5 + (i - 4 * WIDTH)];
-    if (warp == 0) tmem_alloc(&tmem_base, 256);
+    if (warp == 0) tmem_alloc(&tmem_base, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
 
-    if (warp == 8) {
+    if (warp == 16) {
         if (lane == 0) {
-            const uint32_t total = my_tiles * FWD_CHUNKS;
+            const uint32_t total = turns * FWD_CHUNKS;
             uint32_t issued = 0;
             for (uint32_t i = 0; i < total && !abort_flag; i++) {
                 const int s = i % FWD_STAGES;
@@ -560,82 +609,105 @@ __global__ void __launch_bounds__(FWD_THREADS, CTAS) forward_kernel(ForwardArgs 
                     flag_error(g.error, 201, &abort_flag);
                     break;
                 }
-                int layer, kt, half;
-                fwd_chunk(i % FWD_CHUNKS, layer, kt, half);
-                const size_t at = wimg_at(layer) + (size_t)kt * 256 * 128 + (size_t)half * FWD_CHUNK;
                 mbar_expect_tx(&full[s], FWD_CHUNK);
-                bulk_load(ring + (size_t)s * FWD_CHUNK, g.wimg + at, FWD_CHUNK, &full[s]);
+                bulk_load(ring + (size_t)s * FWD_CHUNK, g.wimg + fwd_chunk(i % FWD_CHUNKS), FWD_CHUNK, &full[s]);
                 issued = i + 1;
             }
             for (uint32_t i = issued > (uint32_t)FWD_STAGES ? issued - FWD_STAGES : 0; i < issued; i++)
                 if (!mbar_wait(&full[i % FWD_STAGES], (i / FWD_STAGES) & 1, WAIT_CYCLES))
                     flag_error(g.error, 202, &abort_flag);
         }
-    } else if (warp == 9) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = idesc_bf16(128, 128);
-            uint32_t chunk = 0, acts = 0;
-            const uint32_t act_addr = smem_u32(act), ring_addr = smem_u32(ring);
-            for (uint32_t t = 0; t < my_tiles && !abort_flag; t++) {
-                for (int layer = 0; layer < 4 && !abort_flag; layer++) {
-                    if (!mbar_wait(&act_ready, acts & 1, WAIT_CYCLES)) {
-                        flag_error(g.error, 203, &abort_flag);
-                        break;
-                    }
-                    acts++;
-                    tc_fence_after();
-                    const int n_chunks = layer == 0 ? 2 : 8;
-                    for (int c = 0; c < n_chunks; c++, chunk++) {
-                        const int s = chunk % FWD_STAGES;
-                        if (!mbar_wait(&full[s], (chunk / FWD_STAGES) & 1, WAIT_CYCLES)) {
-                            flag_error(g.error, 204, &abort_flag);
+    } else if (warp >= 17) {
+        // the products of tile t; the two tiles' issuers share the chunks and the tensor pipe, one
+        // issuing while the other waits
+        constexpr uint32_t idesc = idesc_bf16(128, 128);
+        const uint32_t t = warp - 17;
+        const bool leader = elect_one();
+        const uint32_t act_addr = smem_u32(act) + 4 * t * TILE_A, ring_addr = smem_u32(ring), acc = tmem + 256 * t;
+        uint32_t chunk = 0, acts[2] = {0, 0};  // completed waits of act_ready[t][h]
+        bool ok = t < g.per;
+        for (uint32_t i = 0; i < turns && ok; i++) {
+            const bool mine = g.per * (blockIdx.x + i * gridDim.x) + t < g.tiles;  // (else: the chunks pass by)
+            for (int layer = 0; layer < 4 && ok; layer++) {
+                const int kts = layer == 0 ? 1 : 4;
+                for (int c = 0; c < 2 * kts && ok; c++, chunk++) {
+                    const int half = c / kts, kt = c % kts, s = chunk % FWD_STAGES;
+                    if (mine && half == 0 && (kt == 0 || kt == 2)) {  // the activations this k tile begins
+                        ok = __all_sync(0xffffffffu, mbar_wait(&act_ready[t][kt / 2], acts[kt / 2] & 1, WAIT_CYCLES));
+                        acts[kt / 2]++;
+                        if (!ok) {
+                            flag_error(g.error, 203, &abort_flag);
                             break;
                         }
-                        tc_fence_after();
-                        const int kt = layer == 0 ? 0 : c / 2, half = layer == 0 ? c : c % 2;
-                        const uint32_t a_addr = act_addr + kt * TILE_A, b_addr = ring_addr + s * FWD_CHUNK;
+                    }
+                    ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (chunk / FWD_STAGES) & 1, WAIT_CYCLES));
+                    if (!ok) {
+                        flag_error(g.error, 204, &abort_flag);
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t a_addr = act_addr + kt * TILE_A, b_addr = ring_addr + s * FWD_CHUNK;
+                    if (leader) {
+                        if (mine) {
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; k++)
-                            mma_bf16(tmem + 128 * half, sw128_desc(a_addr + 32 * k), sw128_desc(b_addr + 32 * k), idesc,
-                                     (kt | k) != 0);
+                            for (uint32_t k = 0; k < 4; k++)
+                                mma_bf16(acc + 128 * half, sw128_desc(a_addr + 32 * k), sw128_desc(b_addr + 32 * k), idesc, (kt | k) != 0);
+                            if (kt == kts - 1) mma_commit(&acc_ready[t][half]);
+                        }
                         mma_commit(&empty[s]);
                     }
-                    mma_commit(&acc_ready);
+                    __syncwarp();
                 }
             }
         }
     } else {
-        // warps 0-7: inputs, epilogues, outputs; this thread: row r, columns [128 h, 128 h + 128)
-        const uint32_t r = 32 * (warp & 3) + lane, h = warp >> 2;
-        const uint32_t lane_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-        uint32_t accs = 0, dots = 0;
-        for (uint32_t t = 0; t < my_tiles && !__any_sync(0xffffffffu, abort_flag != 0); t++) {
-            const uint32_t tile = blockIdx.x + t * gridDim.x;
+        // the tiles' warps: inputs, epilogues, outputs
+        const uint32_t t = warp >> 3, c = (warp >> 2) & 1, r = 32 * (warp & 3) + lane;
+        const uint32_t lane_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 256 * t;
+        uint8_t *mine = act + 4 * t * TILE_A;
+        uint32_t accs = 0, dots = 0, epilogues = 0;  // layers, tiles and epilogues so far
+        // the two tiles' epilogues take turns (tile 0's n-th, tile 1's n-th, tile 0's next, ...); a tile
+        // alone in the block's last turn does not wait
+        bool paired = false;
+        auto take_turn = [&]() -> bool {
+            const uint32_t n = epilogues++;
+            if (!paired || (t == 0 && n == 0)) return true;
+            return __all_sync(0xffffffffu, mbar_wait(&turn[t], (t == 0 ? n - 1 : n) & 1, WAIT_CYCLES));
+        };
+        auto pass_turn = [&]() {
+            __syncwarp();
+            if (paired && lane == 0) mbar_arrive(&turn[t ^ 1]);
+        };
+        for (uint32_t i = 0; i < turns && !__any_sync(0xffffffffu, abort_flag != 0); i++) {
+            const uint32_t tile = g.per * (blockIdx.x + i * gridDim.x) + t;
+            if (t >= g.per || tile >= g.tiles) break;  // (only the last turn misses a tile)
+            paired = g.per == 2 && tile - t + 1 < g.tiles;
             // candidates: the tile's segment and the point's place in it
             const uint32_t sg = MODE == FWD_CANDIDATES ? segment_of(g, tile) : 0;
             const uint32_t m = MODE == FWD_CANDIDATES ? (tile - g.tile_first[sg]) * 128 + r : tile * 128 + r;
             const uint32_t m_count = MODE == FWD_CANDIDATES ? g.seg[sg].count : g.count;
-            // the inputs: features [32 h, 32 h + 32) of row r of A tile 0 (K = 64)
+            // the inputs: features [32 c, 32 c + 32) of row r of A tile 0 (K = 64)
             uint32_t p[16];
             double u_keep = 1.0;
             uint64_t cand = 0;
             if (MODE == FWD_FROM_X) {
 #pragma unroll
                 for (int e = 0; e < 16; e++) {
-                    const uint32_t k = 32 * h + 2 * e;
+                    const uint32_t k = 32 * c + 2 * e;
                     const float lo = (m < g.count && k < g.inputs) ? g.x[(size_t)m * g.inputs + k] : 0.0f;
                     const float hi = (m < g.count && k + 1 < g.inputs) ? g.x[(size_t)m * g.inputs + k + 1] : 0.0f;
                     p[e] = pack_bf16(lo, hi);
                 }
             } else {
-                // the candidate's phase-space numbers and the subprocess one-hot (the listed candidates
-                // are inside the cuts)
+                // the candidate's phase-space numbers (the first 32 features have them all) and the
+                // subprocess one-hot (the listed candidates are inside the cuts)
                 constexpr int MAXU = pacuda::phase::MAX_UNIFORMS;
                 double u[MAXU];
 #pragma unroll
                 for (int k = 0; k < MAXU; k++) u[k] = 0.0;
                 const uint32_t nx = g.numbers;
-                if (m < m_count) {
+                const bool real = m < m_count;
+                if (real && c == 0) {
                     cand = g.seg[sg].index[m];
                     if (nx == 8) {
                         pacuda::phase::uniforms(g.seg[sg].seed, cand, u);
@@ -647,101 +719,107 @@ __global__ void __launch_bounds__(FWD_THREADS, CTAS) forward_kernel(ForwardArgs 
                     }
                 }
                 u_keep = nx == 8 ? u[8] : u[5];
-                const bool real = m < m_count;
                 const uint32_t family = g.seg[sg].family;
                 float f[32];  // this half's 32 features (constant indices only)
 #pragma unroll
                 for (int k = 0; k < 32; k++) f[k] = 0.0f;
-                if (h == 0 && real) {
+                if (c == 0 && real) {
 #pragma unroll
                     for (int k = 0; k < 8; k++)
                         if ((uint32_t)k < nx) f[k] = (float)u[k];
                 }
 #pragma unroll
                 for (int k = 0; k < 32; k++)
-                    if (real && 32 * h + k == nx + family) f[k] = 1.0f;
+                    if (real && 32 * c + k == nx + family) f[k] = 1.0f;
 #pragma unroll
                 for (int e = 0; e < 16; e++) p[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
             }
 #pragma unroll
             for (int q = 0; q < 4; q++)
-                *reinterpret_cast<uint4 *>(act + sw128_offset(r, 32 * h + 8 * q)) =
+                *reinterpret_cast<uint4 *>(mine + sw128_offset(r, 32 * c + 8 * q)) =
                     make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
             fence_async_shared();
             tc_fence_before();
-            mbar_arrive(&act_ready);
-            float out = 0.0f;
-            bool done = true;
-            for (int layer = 0; layer < 4; layer++) {
-                const bool got = __all_sync(0xffffffffu, mbar_wait(&acc_ready, accs & 1, WAIT_CYCLES));
-                if (!got) {
-                    flag_error(g.error, 205, &abort_flag);
-                    done = false;
-                    break;
-                }
-                accs++;
+            mbar_arrive(&act_ready[t][0]);
+            bool got = true;
+            for (int layer = 0; layer < 3 && got; layer++, accs++) {
+                const float *bias = prm + layer * WIDTH + 64 * c;
+                uint32_t z[4][16], ph[32];
+                got = __all_sync(0xffffffffu, mbar_wait(&acc_ready[t][0], accs & 1, WAIT_CYCLES));
+                if (!got) break;
                 tc_fence_after();
-                const float *bias = prm + layer * WIDTH;  // halved biases (the epilogue works on z / 2)
-                // this half's 128 columns in eight pieces of 16, each piece's tensor-memory load
-                // issued before the previous piece is computed (its latency hidden behind the math)
-                uint32_t buf[2][16];
-                tmem_load16_async(lane_addr + 128 * h, buf[0]);
+                fwd_load(lane_addr + 64 * c, z);
+                if (!(got = take_turn())) break;
+                fwd_activate(z, bias, ph);
+                pass_turn();
+                // (the second half's products have read the activations when they are done)
+                got = __all_sync(0xffffffffu, mbar_wait(&acc_ready[t][1], accs & 1, WAIT_CYCLES));
+                if (!got) break;
+                fwd_store_row(mine + c * TILE_A, r, ph);
+                fence_async_shared();
+                tc_fence_before();
+                mbar_arrive(&act_ready[t][0]);
+                tc_fence_after();
+                fwd_load(lane_addr + 128 + 64 * c, z);
+                if (!(got = take_turn())) break;
+                fwd_activate(z, bias + 128, ph);
+                pass_turn();
+                fwd_store_row(mine + (2 + c) * TILE_A, r, ph);
+                fence_async_shared();
+                tc_fence_before();
+                mbar_arrive(&act_ready[t][1]);
+            }
+            // layer 4 and the output: this thread's half c, its 128 columns in order
+            float out = 0.0f;
+            if (got) got = __all_sync(0xffffffffu, mbar_wait(&acc_ready[t][0], accs & 1, WAIT_CYCLES));
+            if (got && c == 1) got = __all_sync(0xffffffffu, mbar_wait(&acc_ready[t][1], accs & 1, WAIT_CYCLES));
+            uint32_t z[4][16];
+            if (got) {
+                tc_fence_after();
+                fwd_load(lane_addr + 128 * c, z);
+                got = take_turn();
+            }
+            accs++;  // (the first half's threads learn of the second's products from dot_ready)
+            if (!got) {
+                flag_error(g.error, 205, &abort_flag);
+                break;
+            }
 #pragma unroll
-                for (int piece = 0; piece < 8; piece++) {
-                    uint32_t(&cur)[16] = buf[piece & 1];
-                    tmem_wait16(cur);
-                    if (piece + 1 < 8) tmem_load16_async(lane_addr + 128 * h + 16 * (piece + 1), buf[(piece + 1) & 1]);
-                    const int col = 128 * h + 16 * piece;
-                    const float4 *b4 = reinterpret_cast<const float4 *>(bias + col);
-                    float bb[16];
+            for (int part = 0; part < 2; part++) {
+                if (part == 1) fwd_load(lane_addr + 128 * c + 64, z);
+                const float4 *b4 = reinterpret_cast<const float4 *>(prm + 3 * WIDTH + 128 * c + 64 * part);
+                const float4 *w4 = reinterpret_cast<const float4 *>(prm + 4 * WIDTH + 128 * c + 64 * part);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const float4 t4 = b4[q];
-                        bb[4 * q] = t4.x;
-                        bb[4 * q + 1] = t4.y;
-                        bb[4 * q + 2] = t4.z;
-                        bb[4 * q + 3] = t4.w;
-                    }
-                    if (layer < 3) {
-                        uint32_t ph[8];
-#pragma unroll
-                        for (int j = 0; j < 16; j += 2)
-                            ph[j / 2] = pack_bf16(silu_of_half(fmaf(__uint_as_float(cur[j]), 0.5f, bb[j])),
-                                                  silu_of_half(fmaf(__uint_as_float(cur[j + 1]), 0.5f, bb[j + 1])));
-#pragma unroll
-                        for (int q = 0; q < 2; q++)
-                            *reinterpret_cast<uint4 *>(act + (col / 64) * TILE_A + sw128_offset(r, col % 64 + 8 * q)) =
-                                make_uint4(ph[4 * q], ph[4 * q + 1], ph[4 * q + 2], ph[4 * q + 3]);
-                    } else {
-                        const float *w5 = prm + 4 * WIDTH + col;
-#pragma unroll
-                        for (int j = 0; j < 16; j++)
-                            out = fmaf(bf16_round(silu_of_half(fmaf(__uint_as_float(cur[j]), 0.5f, bb[j]))), w5[j], out);
-                    }
-                }
-                if (layer < 3) {
-                    fence_async_shared();
-                    tc_fence_before();
-                    mbar_arrive(&act_ready);
+                for (int q = 0; q < 16; q++) {
+                    uint32_t lo, hi;
+                    fwd_activate4(&z[q / 4][4 * (q % 4)], b4[q], lo, hi);
+                    const float4 ww = w4[q];
+                    out = fmaf(__uint_as_float(lo << 16), ww.x, out);
+                    out = fmaf(__uint_as_float(lo & 0xffff0000u), ww.y, out);
+                    out = fmaf(__uint_as_float(hi << 16), ww.z, out);
+                    out = fmaf(__uint_as_float(hi & 0xffff0000u), ww.w, out);
                 }
             }
+            pass_turn();
+            // (the next tile's inputs are written after both halves of this layer's products: the first
+            // half's threads wait for the second's, which have waited for them)
+            tc_fence_before();
             // the two column halves' dot products meet in shared memory: the upper half's threads
             // write theirs and arrive; the lower half's wait (bounded) and finish the point. The
             // next write of dot_hi comes after this tile's reads: it needs the next tile's inputs,
             // which the lower half writes after them.
-            if (h == 1) {
-                dot_hi[r] = out;
-                mbar_arrive(&dot_ready);
+            if (c == 1) {
+                dot_hi[t][r] = out;
+                mbar_arrive(&dot_ready[t]);
                 continue;
             }
-            const bool have = __all_sync(0xffffffffu, mbar_wait(&dot_ready, dots & 1, WAIT_CYCLES));
+            const bool have = __all_sync(0xffffffffu, mbar_wait(&dot_ready[t], dots & 1, WAIT_CYCLES));
             dots++;
             if (!have) {
                 flag_error(g.error, 206, &abort_flag);
-                continue;
+                break;
             }
-            if (!done) continue;
-            out += dot_hi[r] + prm[5 * WIDTH];
+            out += dot_hi[t][r] + prm[5 * WIDTH];
             if (MODE == FWD_FROM_X) {
                 if (m < g.count) g.out[m] = out;
             } else {
@@ -768,7 +846,7 @@ __global__ void __launch_bounds__(FWD_THREADS, CTAS) forward_kernel(ForwardArgs 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) tmem_dealloc(tmem, 256);
+    if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 // ---- host ---------------------------------------------------------------------------------------
@@ -797,16 +875,14 @@ bool launch_gemm(const GemmArgs &g, uint32_t m_tiles, uint32_t splits, cudaStrea
     return !failed(cudaGetLastError(), "product kernel launch");
 }
 
-// blocks per SM of the inference kernel: 2 (two blocks, a 2-stage weight ring each) or 1 (one
-// block, a 9-stage ring)
-int g_forward_blocks = 2;
+// tiles in flight per SM of the inference kernel: 2 or 1
+int g_forward_tiles = 2;
 
-template <int MODE, int CTAS>
-bool launch_forward_shape(const ForwardArgs &g, cudaStream_t s) {
+template <int MODE>
+bool launch_forward(ForwardArgs &g, cudaStream_t s) {
     static bool configured = false;
     if (!configured) {
-        if (failed(cudaFuncSetAttribute(forward_kernel<MODE, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        FwdShape<CTAS>::SMEM),
+        if (failed(cudaFuncSetAttribute(forward_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM),
                    "inference kernel attributes"))
             return false;
         configured = true;
@@ -814,15 +890,12 @@ bool launch_forward_shape(const ForwardArgs &g, cudaStream_t s) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint32_t grid = std::min<uint32_t>(g.tiles, (uint32_t)CTAS * (uint32_t)sms);
-    forward_kernel<MODE, CTAS><<<grid, FWD_THREADS, FwdShape<CTAS>::SMEM, s>>>(g);
+    // pairs of tiles once there are more tiles than SMs (a pair takes less than two turns of one)
+    g.per = g_forward_tiles == 2 && g.tiles > (uint32_t)sms ? 2 : 1;
+    const uint32_t grid = std::min<uint32_t>((g.tiles + g.per - 1) / g.per, (uint32_t)sms);
+    forward_kernel<MODE><<<grid, FWD_THREADS, FWD_SMEM, s>>>(g);
     g_last_launches++;
     return !failed(cudaGetLastError(), "inference launch");
-}
-
-template <int MODE>
-bool launch_forward(const ForwardArgs &g, cudaStream_t s) {
-    return g_forward_blocks == 1 ? launch_forward_shape<MODE, 1>(g, s) : launch_forward_shape<MODE, 2>(g, s);
 }
 
 }  // namespace
@@ -871,7 +944,7 @@ extern "C" uint32_t pacuda_sg_last_launches(void) { return g_last_launches; }
 
 extern "C" int pacuda_sg_set_inference_blocks(uint32_t blocks) {
     if (blocks != 1 && blocks != 2) return ST_INVALID;
-    g_forward_blocks = (int)blocks;
+    g_forward_tiles = (int)blocks;
     return ST_OK;
 }
 

@@ -44,6 +44,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
 }
 // A wait on phase `parity` of `bar` that gives up after about `cycles` SM clock cycles (false).
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long long cycles) {
+    if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try_wait(bar, parity))
         if (clock64() - t0 > cycles) return false;
@@ -134,6 +135,22 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
 // instruction descriptor of kind::f16: A and B BF16, D FP32, both K-major, M x N
 __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
+}
+
+// The warp's index in a form the compiler knows to be the same for all its lanes, and one lane of
+// the warp. A warp that issues products goes through its loop as a whole, its elected lane alone
+// executing the issuing instructions: their operands are then in uniform registers, where a loop
+// of one lane made the compiler broadcast each operand of each product (about 30 instructions per
+// product, 200 cycles beside the 64 that the product takes).
+__device__ __forceinline__ uint32_t uniform_warp() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(p));
+    return p != 0;
 }
 
 // D[tmem] (+)= A * B^T for one K step of 16; issued by one thread

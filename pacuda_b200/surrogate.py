@@ -116,7 +116,7 @@ class Network:
 
 
 def set_inference_blocks(blocks):
-    """Blocks per SM of the fused inference kernel (1 or 2)."""
+    """Tiles of points in flight per SM in the fused inference kernel (1 or 2)."""
     _check(lib().pacuda_sg_set_inference_blocks(int(blocks)), "set_inference_blocks")
 
 
