@@ -7,13 +7,13 @@
 // image (the N side) is one row tile of N rows (64 or 256) as K/64 tiles of N x 64 values. One
 // bulk copy moves one tile into shared memory in the layout the tensor cores read.
 //
-// Training (one batch of B points, B a multiple of 128):
-//   forward   H_l = silu(Z_l), Z_l = H_{l-1} W_l^T + b_l     A = H_{l-1} image, B = W_l image
-//   layer 4   out = w5 . bf16(h4) + b5, dout = 2 (out - y) / B, dZ4 = dout w5 silu'(z4) in the epilogue
-//   backward  dZ_{l-1} = (dZ_l W_l) silu'(Z_{l-1})               A = dZ_l image, B = W_l^T image
-//             dW_l = dZ_l^T H_{l-1} (split over the batch)       A = dZ_l^T image, B = H_{l-1}^T image
-// Every product is C = A B^T with both operands K-major, so one kernel serves all of them; the
-// epilogues write the transposed images the later products need.
+// Training (one batch of B points, B a multiple of 128), three launches:
+//   chain_kernel   per 128 points, the forward products H_l = silu(H_{l-1} W_l^T + b_l), the output
+//                  layer and dZ4, then the backward products dZ_{l-1} = (dZ_l W_l) silu'(Z_{l-1}),
+//                  each layer's operand in shared memory; it writes X, H_l and dZ_l as A images
+//   dw_kernel      dW_l = dZ_l^T H_{l-1}, split over the batch: the same images with K along the
+//                  points (MN-major operands, so no transposed copy of them is written or read)
+//   update_kernel  the sums of the partials in a fixed order, Adam and the weight images
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -51,7 +51,6 @@ __host__ __device__ constexpr size_t wimg_at(int layer) {
     return layer == 0 ? WIMG_L1 : layer == 1 ? WIMG_L2 : layer == 2 ? WIMG_L3 : WIMG_L4;
 }
 
-enum Epi { EPI_PARTIAL, EPI_HIDDEN, EPI_LAST, EPI_BACK };
 enum Status { ST_OK = 0, ST_INVALID = 2, ST_DEVICE = 3 };
 
 // ---- arithmetic shared by every kernel --------------------------------------------------------
@@ -71,11 +70,6 @@ __device__ __forceinline__ float silu_grad(float z) {
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t *>(&v);
-}
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-// byte offset of element (r, k) in an A image whose row tiles hold `kt` tiles of 64 values of K
-__device__ __forceinline__ size_t a_img(uint32_t r, uint32_t k, uint32_t kt) {
-    return ((size_t)(r >> 7) * kt + (k >> 6)) * TILE_A + sw128_offset(r & 127u, k & 63u);
 }
 // byte offset of element (r, k) in a B image of `rows` rows
 __device__ __forceinline__ size_t b_img(uint32_t r, uint32_t k, uint32_t rows) {
@@ -103,65 +97,347 @@ __device__ __forceinline__ void flag_error(int *error, int code, volatile int *a
     *abort_flag = 1;
 }
 
-// ---- the product kernel --------------------------------------------------------------------------
+// ---- the forward and backward chain -------------------------------------------------------------
+//
+// One block per 128 points at a time: seven products (four layers forward, three back) one after the
+// other, each on the operand that the epilogue before it left in shared memory. Warps 0-15 run the
+// epilogues: thread (quarter, lane, c) owns point r = 32 quarter + lane, tensor-memory lane r, and
+// the 64 columns of quarter c; warp 16 streams the weight images (32 KB chunks: a k tile of all 256
+// rows), warp 17 issues the products (M = 128, N = 256). Z stays with the thread that made it: it
+// goes to global memory and back in the order of the threads.
+//
+// At the training batch (16 384 points, 128 blocks) the chain of products and epilogues is what
+// bounds it: a product is 2 048 cycles of the tensor pipe, an epilogue as many of the MUFU (a tanh
+// per value). As seven launches, each with its operands read from and written to global memory, its
+// transposed copies stored in 2-byte pieces and four epilogue warps, this part took 127 us of a
+// step's 206; here 35 of 69 (68 thousand cycles per tile: 3 to 4 for each product with its operand's
+// hand-over, 4.5 to 5 for an epilogue, 11 for the output layer's).
 
-struct GemmArgs {
-    const uint8_t *a;  // A image
-    const uint8_t *b;  // B image (N rows)
-    uint32_t k_tiles;  // tiles of K this block multiplies (its split)
-    uint32_t a_kt;     // tiles of K per row tile of the whole A image
-    // EPI_PARTIAL: partial[(split * M + m) * N + n]
-    float *partial;
-    uint32_t m_rows;   // M
-    // hidden layers
-    const float *bias;
-    uint8_t *h_img;    // next A image (K = 256)
-    uint8_t *ht_img;   // H^T as a B image of 256 rows, K = batch
-    __nv_bfloat16 *z;  // [batch][256]
-    // backward
-    const __nv_bfloat16 *zprev;  // [batch][256]
-    uint8_t *dz_img;   // dZ as an A image (K = 256)
-    uint8_t *dzt_img;  // dZ^T as an A image of 256 rows (K = batch)
-    float *db_partial;      // [block][256]
-    // layer 4
-    const float *w5, *b5, *y;
+constexpr int CH_EPI = 512, CH_THREADS = CH_EPI + 64, CH_STAGES = 4;
+constexpr uint32_t CH_CHUNK = 256 * 128;  // 32 KB
+constexpr uint32_t CH_SMEM = 4 * TILE_A + CH_STAGES * CH_CHUNK + 1024;
+constexpr int CH_CHUNKS = 1 + 6 * 4;  // per tile: layer 1 (1 k tile), layers 2-4 and back (4 each)
+
+struct ChainArgs {
+    const uint8_t *wimg, *wtimg;
+    const float *params, *x, *y;
+    uint32_t inputs, tiles;
     float inv_batch;
-    float *dw5_partial;     // [block][256]
-    float *scalar_partial;  // [block][2]: sum dout, sum (out - y)^2
-    uint32_t batch;
+    uint8_t *x_img, *h_img[3], *dz_img[4];
+    uint4 *z[3];             // [tile][8][thread]: 8 BF16 values each
+    float *db[4];            // [tile][256]
+    float *dw5;              // [tile][256]
+    float *scalars;          // [tile][2]: sum dout, sum (out - y)^2
     int *error;
 };
 
-template <int N>
-struct GemmShape {
-    static constexpr uint32_t A_BYTES = TILE_A, B_BYTES = N * 128u, STAGE = A_BYTES + B_BYTES;
-    static constexpr int STAGES = N == 256 ? 4 : 6;
-    static constexpr uint32_t SMEM = STAGES * STAGE + 1024;  // + alignment of the first tile
-};
-
-// column sums of the block's 128 rows for the 32 columns of chunk c: warp sums into `part`
-__device__ __forceinline__ void column_chunk(float (&v)[32], float (*part)[WIDTH], int c) {
-    const float s = warp_column_sum(v);
-    part[threadIdx.x >> 5][32 * c + (threadIdx.x & 31)] = s;
+// row r of one A tile from 32 packed pairs
+__device__ __forceinline__ void store_row(uint8_t *tile, uint32_t r, const uint32_t (&ph)[32]) {
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        *reinterpret_cast<uint4 *>(tile + sw128_offset(r, 8 * q)) =
+            make_uint4(ph[4 * q], ph[4 * q + 1], ph[4 * q + 2], ph[4 * q + 3]);
 }
 
-template <int N, int EPI>
-__global__ void __launch_bounds__(128, 1) gemm_kernel(GemmArgs g) {
-    using S = GemmShape<N>;
+__device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+
+__global__ void __launch_bounds__(CH_THREADS, 1) chain_kernel(ChainArgs g) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full[S::STAGES], empty[S::STAGES], done;
+    __shared__ uint64_t full[CH_STAGES], empty[CH_STAGES], act_ready, acc_ready;
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
-    __shared__ float part_a[4][WIDTH], part_b[4][WIDTH];
-    __shared__ float scal[4][2];
+    __shared__ __align__(16) float bias[4][WIDTH], w5[WIDTH + 4];
+    __shared__ float part_a[4][WIDTH], part_b[4][WIDTH], dot[4][128], scal[4][2];
+    const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
+    uint8_t *act = smem_raw + pad, *ring = act + 4 * TILE_A;
+    const int warp = (int)uniform_warp(), lane = threadIdx.x & 31;
+    const uint32_t turns = blockIdx.x < g.tiles ? (g.tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < CH_STAGES; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(&act_ready, 1);
+        mbar_init(&acc_ready, 1);
+        abort_flag = 0;
+        fence_mbar_init();
+    }
+    for (int i = threadIdx.x; i < 4 * WIDTH; i += CH_THREADS) bias[i / WIDTH][i % WIDTH] = g.params[bias_at(i / WIDTH) + i % WIDTH];
+    for (int i = threadIdx.x; i <= WIDTH; i += CH_THREADS) w5[i] = g.params[P_W5 + i];  // (then b5)
+    if (warp == 0) tmem_alloc(&tmem_base, 256);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+
+    if (warp == 16) {
+        if (lane == 0) {
+            const uint32_t total = turns * CH_CHUNKS;
+            uint32_t issued = 0;
+            for (uint32_t i = 0; i < total && !abort_flag; i++) {
+                const int s = i % CH_STAGES;
+                if (i >= (uint32_t)CH_STAGES && !mbar_wait(&empty[s], ((i / CH_STAGES) - 1) & 1, WAIT_CYCLES)) {
+                    flag_error(g.error, 101, &abort_flag);
+                    break;
+                }
+                const uint32_t c = i % CH_CHUNKS;
+                // forward: W1, W2, W3, W4; back: the transposes of W4, W3, W2
+                const uint8_t *src = c < 13 ? g.wimg + (size_t)c * CH_CHUNK
+                                            : g.wtimg + (size_t)(2 - (c - 13) / 4) * 4 * CH_CHUNK + (c - 13) % 4 * CH_CHUNK;
+                mbar_expect_tx(&full[s], CH_CHUNK);
+                bulk_load(ring + (size_t)s * CH_CHUNK, src, CH_CHUNK, &full[s]);
+                issued = i + 1;
+            }
+            // the copies still in flight end before the block does
+            for (uint32_t i = issued > (uint32_t)CH_STAGES ? issued - CH_STAGES : 0; i < issued; i++)
+                if (!mbar_wait(&full[i % CH_STAGES], (i / CH_STAGES) & 1, WAIT_CYCLES)) flag_error(g.error, 102, &abort_flag);
+        }
+    } else if (warp == 17) {
+        constexpr uint32_t idesc = idesc_bf16(128, 256);
+        const bool leader = elect_one();
+        const uint32_t act_addr = smem_u32(act), ring_addr = smem_u32(ring);
+        uint32_t chunk = 0;
+        bool ok = true;
+        for (uint32_t n = 0; n < 7 * turns && ok; n++) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&act_ready, n & 1, WAIT_CYCLES));
+            if (!ok) {
+                flag_error(g.error, 103, &abort_flag);
+                break;
+            }
+            const int kts = n % 7 == 0 ? 1 : 4;
+            for (int kt = 0; kt < kts; kt++, chunk++) {
+                const int s = chunk % CH_STAGES;
+                ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (chunk / CH_STAGES) & 1, WAIT_CYCLES));
+                if (!ok) {
+                    flag_error(g.error, 104, &abort_flag);
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t a_addr = act_addr + kt * TILE_A, b_addr = ring_addr + s * CH_CHUNK;
+                if (leader) {
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++)
+                        mma_bf16(tmem, sw128_desc(a_addr + 32 * k), sw128_desc(b_addr + 32 * k), idesc, (kt | k) != 0);
+                    mma_commit(&empty[s]);
+                    if (kt == kts - 1) mma_commit(&acc_ready);
+                }
+                __syncwarp();
+            }
+        }
+    } else {
+        const uint32_t c = warp >> 2, quarter = warp & 3, r = 32 * quarter + lane, col = 64 * c;
+        const uint32_t acc = tmem + ((uint32_t)(32 * quarter) << 16) + col;
+        const bool first = threadIdx.x == 0;
+        uint8_t *mine = act + c * TILE_A;  // this thread's columns are one A tile's
+        uint32_t accs = 0;
+        // After a given-up wait the threads go on without waiting (every barrier is met; the outputs
+        // are not used: the error is flagged).
+        auto wait_acc = [&]() {
+            if (!abort_flag && !mbar_wait(&acc_ready, accs & 1, WAIT_CYCLES)) flag_error(g.error, 105, &abort_flag);
+            accs++;
+            __syncwarp();
+            tc_fence_after();
+            // the activations' stores have read them: the epilogue may replace them
+            if (first) bulk_store_read();
+            epilogue_barrier();
+        };
+        // the written operand is stored to `image` and, with `next`, handed to the next product
+        auto hand_over = [&](uint8_t *image, uint32_t bytes, bool next) {
+            fence_async_shared();
+            tc_fence_before();
+            epilogue_barrier();
+            if (first) {
+                if (next) mbar_arrive(&act_ready);
+                bulk_store(image, act, bytes);
+            }
+        };
+        // the rows' sums of the 128 points, from the quarters' sums, into `out` [tile][256]
+        auto column_sums = [&](float (*part)[WIDTH], float *out, uint32_t tile) {
+            if (threadIdx.x < WIDTH)
+                out[(size_t)tile * WIDTH + threadIdx.x] =
+                    part[0][threadIdx.x] + part[1][threadIdx.x] + part[2][threadIdx.x] + part[3][threadIdx.x];
+        };
+        for (uint32_t i = 0; i < turns; i++) {
+            const uint32_t tile = blockIdx.x + i * gridDim.x, m = tile * 128 + r;
+            uint32_t ph[32];
+            // the inputs: features [16 c, 16 c + 16) of row r (K = 64)
+            {
+                if (first) bulk_store_read();  // (the last tile's dZ1)
+                epilogue_barrier();
+                uint32_t p[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const uint32_t k = 16 * c + 2 * e;
+                    const float lo = k < g.inputs ? g.x[(size_t)m * g.inputs + k] : 0.0f;
+                    const float hi = k + 1 < g.inputs ? g.x[(size_t)m * g.inputs + k + 1] : 0.0f;
+                    p[e] = pack_bf16(lo, hi);
+                }
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                    *reinterpret_cast<uint4 *>(act + sw128_offset(r, 16 * c + 8 * q)) =
+                        make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
+                hand_over(g.x_img + (size_t)tile * TILE_A, TILE_A, true);
+            }
+            // layers 1-3 forward
+            for (int layer = 0; layer < 3; layer++) {
+                wait_acc();
+                uint4 *zt = g.z[layer] + (size_t)tile * 8 * CH_EPI + threadIdx.x;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    float v[32];
+                    uint32_t pz[16];
+                    tmem_load32(acc + 32 * h, v);
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        const float z0 = v[j] + bias[layer][col + 32 * h + j], z1 = v[j + 1] + bias[layer][col + 32 * h + j + 1];
+                        pz[j / 2] = pack_bf16(z0, z1);
+                        ph[16 * h + j / 2] = pack_bf16(silu(z0), silu(z1));
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        zt[(4 * h + q) * CH_EPI] = make_uint4(pz[4 * q], pz[4 * q + 1], pz[4 * q + 2], pz[4 * q + 3]);
+                }
+                store_row(mine, r, ph);
+                hand_over(g.h_img[layer] + (size_t)tile * 4 * TILE_A, 4 * TILE_A, true);
+            }
+            // layer 4 and the output layer: out, dout, dZ4 = dout w5 silu'(z4)
+            wait_acc();
+            {
+                float out = 0.0f;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    float v[32];
+                    tmem_load32(acc + 32 * h, v);
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        const int n = col + 32 * h + j;
+                        const uint32_t w = pack_bf16(silu(v[j] + bias[3][n]), silu(v[j + 1] + bias[3][n + 1]));
+                        out += __uint_as_float(w << 16) * w5[n];
+                        out += __uint_as_float(w & 0xffff0000u) * w5[n + 1];
+                    }
+                }
+                dot[c][r] = out;
+                epilogue_barrier();
+                out = dot[0][r] + dot[1][r] + dot[2][r] + dot[3][r] + w5[WIDTH];
+                const float err = out - g.y[m], dout = 2.0f * err * g.inv_batch;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    float v[32], hw[32];
+                    tmem_load32(acc + 32 * h, v);
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {
+                        const int n = col + 32 * h + j;
+                        const float z = v[j] + bias[3][n], t = tanh_fast(0.5f * z), s = 0.5f + 0.5f * t;
+                        hw[j] = fmaf(0.5f * z, t, 0.5f * z);
+                        v[j] = dout * w5[n] * (s * (1.0f + z * (1.0f - s)));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        ph[16 * h + j / 2] = pack_bf16(v[j], v[j + 1]);
+                        const uint32_t w = pack_bf16(hw[j], hw[j + 1]);
+                        hw[j] = dout * __uint_as_float(w << 16);
+                        hw[j + 1] = dout * __uint_as_float(w & 0xffff0000u);
+                    }
+                    part_a[quarter][col + 32 * h + lane] = warp_column_sum(v);
+                    part_b[quarter][col + 32 * h + lane] = warp_column_sum(hw);
+                }
+                if (c == 0) {
+                    float a = dout, b = err * err;
+#pragma unroll
+                    for (int off = 16; off >= 1; off >>= 1) {
+                        a += __shfl_xor_sync(0xffffffffu, a, off);
+                        b += __shfl_xor_sync(0xffffffffu, b, off);
+                    }
+                    if (lane == 0) {
+                        scal[quarter][0] = a;
+                        scal[quarter][1] = b;
+                    }
+                }
+                store_row(mine, r, ph);
+                hand_over(g.dz_img[3] + (size_t)tile * 4 * TILE_A, 4 * TILE_A, true);
+                column_sums(part_a, g.db[3], tile);
+                column_sums(part_b, g.dw5, tile);
+                if (threadIdx.x < 2)
+                    g.scalars[2 * tile + threadIdx.x] =
+                        scal[0][threadIdx.x] + scal[1][threadIdx.x] + scal[2][threadIdx.x] + scal[3][threadIdx.x];
+            }
+            // back: dZ3, dZ2, dZ1
+            for (int layer = 2; layer >= 0; layer--) {
+                uint4 zs[8];
+                const uint4 *zt = g.z[layer] + (size_t)tile * 8 * CH_EPI + threadIdx.x;
+#pragma unroll
+                for (int q = 0; q < 8; q++) zs[q] = zt[q * CH_EPI];
+                wait_acc();
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    float v[32];
+                    tmem_load32(acc + 32 * h, v);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const uint32_t ws[4] = {zs[4 * h + q].x, zs[4 * h + q].y, zs[4 * h + q].z, zs[4 * h + q].w};
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            v[8 * q + 2 * e] *= silu_grad(__uint_as_float(ws[e] << 16));
+                            v[8 * q + 2 * e + 1] *= silu_grad(__uint_as_float(ws[e] & 0xffff0000u));
+                            ph[16 * h + 4 * q + e] = pack_bf16(v[8 * q + 2 * e], v[8 * q + 2 * e + 1]);
+                        }
+                    }
+                    part_a[quarter][col + 32 * h + lane] = warp_column_sum(v);
+                }
+                store_row(mine, r, ph);
+                hand_over(g.dz_img[layer] + (size_t)tile * 4 * TILE_A, 4 * TILE_A, layer > 0);
+                column_sums(part_a, g.db[layer], tile);
+            }
+        }
+        if (first) bulk_store_done();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0) tmem_dealloc(tmem, 256);
+}
+
+// ---- the weight gradients -------------------------------------------------------------------------
+//
+// dW_l = dZ_l^T H_{l-1}: a block takes one layer's upper or lower 128 rows over a part of the batch,
+// 128 points per stage, A = dZ's tiles of those rows and B = H's (X's) tiles, K along the points. The
+// parts fill the chip once (148 blocks for more than 20 tiles of points); FP32 partials go out as
+// [part][column / 4][row][4], so that a warp writes whole lines.
+
+constexpr uint32_t DW_PARTS = 21, DW_PARTS_X = 11;  // parts of the batch, layers 2-4 and layer 1
+constexpr uint32_t DW_STAGE = 6 * TILE_A, DW_SMEM = 2 * DW_STAGE + 1024;
+inline __host__ __device__ uint32_t dw_parts(int layer, uint32_t tiles) {
+    const uint32_t most = layer == 0 ? DW_PARTS_X : DW_PARTS;
+    return tiles < most ? tiles : most;
+}
+
+struct DwArgs {
+    const uint8_t *x_img, *h_img[3], *dz_img[4];
+    float *partial[4];
+    uint32_t tiles;
+    int *error;
+};
+
+__global__ void __launch_bounds__(256, 1) dw_kernel(DwArgs g) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t full[2], empty[2], done;
+    __shared__ uint32_t tmem_base;
+    __shared__ volatile int abort_flag;
     const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
     uint8_t *smem = smem_raw + pad;
     const int warp = (int)uniform_warp(), lane = threadIdx.x & 31;
-    const uint32_t mt = blockIdx.x, split = blockIdx.y;
-    constexpr uint32_t COLS = N < 32 ? 32 : N;
+    // the block's layer, rows and part: layers 2-4 first
+    const uint32_t parts = dw_parts(1, g.tiles), parts_x = dw_parts(0, g.tiles);
+    uint32_t b = blockIdx.x;
+    const int layer = b < 6 * parts ? 1 + (int)(b / (2 * parts)) : 0;
+    b = layer ? b % (2 * parts) : b - 6 * parts;
+    const uint32_t mine = layer ? parts : parts_x, half = b / mine, part = b % mine;
+    const uint32_t t0 = g.tiles * part / mine, t1 = g.tiles * (part + 1) / mine;
+    const uint32_t width = layer ? WIDTH : IN, b_bytes = width / 64 * TILE_A, bytes = 2 * TILE_A + b_bytes;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S::STAGES; s++) {
+        for (int s = 0; s < 2; s++) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
@@ -169,48 +445,46 @@ __global__ void __launch_bounds__(128, 1) gemm_kernel(GemmArgs g) {
         abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 0) tmem_alloc(&tmem_base, COLS);
+    if (warp == 0) tmem_alloc(&tmem_base, 256);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
-    const uint8_t *a_base = g.a + ((size_t)mt * g.a_kt + (size_t)split * g.k_tiles) * S::A_BYTES;
-    const uint8_t *b_base = g.b + (size_t)split * g.k_tiles * S::B_BYTES;
-
-    if (warp == 0 && lane == 0) {
-        // producer: the tiles of A and B into the stage ring
-        uint32_t issued = 0;
-        for (uint32_t i = 0; i < g.k_tiles && !abort_flag; i++) {
-            const int s = i % S::STAGES;
-            if (i >= (uint32_t)S::STAGES && !mbar_wait(&empty[s], ((i / S::STAGES) - 1) & 1, WAIT_CYCLES)) {
-                flag_error(g.error, 101, &abort_flag);
-                break;
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint8_t *a = g.dz_img[layer] + 2 * half * TILE_A, *h = layer ? g.h_img[layer - 1] : g.x_img;
+            uint32_t issued = 0;
+            for (uint32_t i = 0; i < t1 - t0 && !abort_flag; i++) {
+                const int s = i & 1;
+                if (i >= 2 && !mbar_wait(&empty[s], ((i >> 1) - 1) & 1, WAIT_CYCLES)) {
+                    flag_error(g.error, 111, &abort_flag);
+                    break;
+                }
+                uint8_t *st = smem + s * DW_STAGE;
+                mbar_expect_tx(&full[s], bytes);
+                bulk_load(st, a + (size_t)(t0 + i) * 4 * TILE_A, 2 * TILE_A, &full[s]);
+                bulk_load(st + 2 * TILE_A, h + (size_t)(t0 + i) * b_bytes, b_bytes, &full[s]);
+                issued = i + 1;
             }
-            uint8_t *st = smem + (size_t)s * S::STAGE;
-            mbar_expect_tx(&full[s], S::STAGE);
-            bulk_load(st, a_base + (size_t)i * S::A_BYTES, S::A_BYTES, &full[s]);
-            bulk_load(st + S::A_BYTES, b_base + (size_t)i * S::B_BYTES, S::B_BYTES, &full[s]);
-            issued = i + 1;
+            for (uint32_t i = issued > 2 ? issued - 2 : 0; i < issued; i++)
+                if (!mbar_wait(&full[i & 1], (i >> 1) & 1, WAIT_CYCLES)) flag_error(g.error, 112, &abort_flag);
         }
-        // the copies still in flight end before the block does
-        for (uint32_t i = issued > (uint32_t)S::STAGES ? issued - S::STAGES : 0; i < issued; i++)
-            if (!mbar_wait(&full[i % S::STAGES], (i / S::STAGES) & 1, WAIT_CYCLES)) flag_error(g.error, 102, &abort_flag);
     } else if (warp == 1) {
-        // the MMA issuer: 4 steps of K = 16 per tile
-        constexpr uint32_t idesc = idesc_bf16(128, N);
+        const uint32_t idesc = (layer ? idesc_bf16(128, WIDTH) : idesc_bf16(128, IN)) | IDESC_MN;
         const bool leader = elect_one();
-        for (uint32_t i = 0; i < g.k_tiles; i++) {
-            const int s = i % S::STAGES;
-            if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (i / S::STAGES) & 1, WAIT_CYCLES))) {
-                flag_error(g.error, 103, &abort_flag);
+        for (uint32_t i = 0; i < t1 - t0; i++) {
+            const int s = i & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (i >> 1) & 1, WAIT_CYCLES))) {
+                flag_error(g.error, 113, &abort_flag);
                 break;
             }
             tc_fence_after();
-            const uint32_t a_addr = smem_u32(smem) + s * S::STAGE, b_addr = a_addr + S::A_BYTES;
+            const uint32_t a_addr = smem_u32(smem) + s * DW_STAGE, b_addr = a_addr + 2 * TILE_A;
             if (leader) {
 #pragma unroll
-                for (uint32_t k = 0; k < 4; k++)
-                    mma_bf16(tmem, sw128_desc(a_addr + 32 * k), sw128_desc(b_addr + 32 * k), idesc, (i | k) != 0);
+                for (uint32_t k = 0; k < 8; k++)  // 16 points each
+                    mma_bf16(tmem, sw128_mn_desc(a_addr + 2048 * k, TILE_A), sw128_mn_desc(b_addr + 2048 * k, TILE_A), idesc,
+                             (i | k) != 0);
                 mma_commit(&empty[s]);
             }
             __syncwarp();
@@ -218,157 +492,26 @@ __global__ void __launch_bounds__(128, 1) gemm_kernel(GemmArgs g) {
         if (leader) mma_commit(&done);
     }
     __syncwarp();
-    // warp-uniform from here on: the tensor-memory loads below are .sync.aligned
     bool ready = mbar_wait(&done, 0, WAIT_CYCLES);
     tc_fence_after();
-    if (!ready) flag_error(g.error, 104, &abort_flag);
+    if (!ready) flag_error(g.error, 114, &abort_flag);
     ready = __all_sync(0xffffffffu, ready && !abort_flag);
-
-    const uint32_t r = 32 * warp + lane;  // this thread's row of the tile (its tensor-memory lane)
-    const uint32_t m = mt * 128 + r;
-    const uint32_t lane_addr = tmem + ((uint32_t)(32 * warp) << 16);
     if (ready) {
-        float v[32];
-        if (EPI == EPI_PARTIAL) {
-            float *dst = g.partial + ((size_t)split * g.m_rows + m) * N;
-            for (int c = 0; c < N / 32; c++) {
-                tmem_load32(lane_addr + 32 * c, v);
-                float4 *d4 = reinterpret_cast<float4 *>(dst + 32 * c);
+        const uint32_t quarter = warp & 3, m = 128 * half + 32 * quarter + lane;
+        const uint32_t columns = width / 2, col = columns * (warp >> 2);  // this warp's columns
+        float4 *out = reinterpret_cast<float4 *>(g.partial[layer]) + (size_t)part * width / 4 * WIDTH + m;
+        for (uint32_t c = col; c < col + columns; c += 32) {
+            float v[32];
+            tmem_load32(tmem + ((32 * quarter) << 16) + c, v);
 #pragma unroll
-                for (int q = 0; q < 8; q++) d4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            }
-        } else if (EPI == EPI_HIDDEN) {
-            for (int c = 0; c < WIDTH / 32; c++) {
-                tmem_load32(lane_addr + 32 * c, v);
-                uint32_t ph[16], pz[16];
-#pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    const float z0 = v[j] + g.bias[32 * c + j], z1 = v[j + 1] + g.bias[32 * c + j + 1];
-                    pz[j / 2] = pack_bf16(z0, z1);
-                    ph[j / 2] = pack_bf16(silu(z0), silu(z1));
-                }
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    *reinterpret_cast<uint4 *>(g.h_img + a_img(m, 32 * c + 8 * q, 4)) =
-                        make_uint4(ph[4 * q], ph[4 * q + 1], ph[4 * q + 2], ph[4 * q + 3]);
-                    reinterpret_cast<uint4 *>(g.z + (size_t)m * WIDTH + 32 * c)[q] =
-                        make_uint4(pz[4 * q], pz[4 * q + 1], pz[4 * q + 2], pz[4 * q + 3]);
-                }
-#pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const uint32_t w = ph[j / 2];
-                    const uint16_t bits = (uint16_t)(j & 1 ? w >> 16 : w & 0xffff);
-                    *reinterpret_cast<uint16_t *>(g.ht_img + b_img(32 * c + j, m, WIDTH)) = bits;
-                }
-            }
-        } else {
-            // EPI_LAST and EPI_BACK: dZ, its transpose and the column sums
-            float dout = 0.0f, err = 0.0f;
-            if (EPI == EPI_LAST) {
-                float out = 0.0f;
-                for (int c = 0; c < WIDTH / 32; c++) {
-                    tmem_load32(lane_addr + 32 * c, v);
-#pragma unroll
-                    for (int j = 0; j < 32; j++) out += bf16_round(silu(v[j] + g.bias[32 * c + j])) * g.w5[32 * c + j];
-                }
-                out += g.b5[0];
-                err = out - g.y[m];
-                dout = 2.0f * err * g.inv_batch;
-            }
-            const uint32_t batch_kt = g.batch / 64;
-            for (int c = 0; c < WIDTH / 32; c++) {
-                tmem_load32(lane_addr + 32 * c, v);
-                float dz[32], hw[32];
-                if (EPI == EPI_LAST) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const int n = 32 * c + j;
-                        const float z = v[j] + g.bias[n];
-                        hw[j] = dout * bf16_round(silu(z));
-                        dz[j] = dout * g.w5[n] * silu_grad(z);
-                    }
-                } else {
-                    const uint4 *zp = reinterpret_cast<const uint4 *>(g.zprev + (size_t)m * WIDTH + 32 * c);
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const uint4 w = zp[q];
-                        const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const float lo = __uint_as_float(ws[e] << 16), hi = __uint_as_float(ws[e] & 0xffff0000u);
-                            dz[8 * q + 2 * e] = v[8 * q + 2 * e] * silu_grad(lo);
-                            dz[8 * q + 2 * e + 1] = v[8 * q + 2 * e + 1] * silu_grad(hi);
-                        }
-                    }
-                }
-                uint32_t pd[16];
-#pragma unroll
-                for (int j = 0; j < 32; j += 2) pd[j / 2] = pack_bf16(dz[j], dz[j + 1]);
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    *reinterpret_cast<uint4 *>(g.dz_img + a_img(m, 32 * c + 8 * q, 4)) =
-                        make_uint4(pd[4 * q], pd[4 * q + 1], pd[4 * q + 2], pd[4 * q + 3]);
-#pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const uint32_t w = pd[j / 2];
-                    const uint16_t bits = (uint16_t)(j & 1 ? w >> 16 : w & 0xffff);
-                    *reinterpret_cast<uint16_t *>(g.dzt_img + a_img(32 * c + j, m, batch_kt)) = bits;
-                }
-                column_chunk(dz, part_a, c);
-                if (EPI == EPI_LAST) column_chunk(hw, part_b, c);
-            }
-            if (EPI == EPI_LAST) {
-                float a = dout, b = err * err;
-#pragma unroll
-                for (int off = 16; off >= 1; off >>= 1) {
-                    a += __shfl_xor_sync(0xffffffffu, a, off);
-                    b += __shfl_xor_sync(0xffffffffu, b, off);
-                }
-                if (lane == 0) {
-                    scal[warp][0] = a;
-                    scal[warp][1] = b;
-                }
-            }
+            for (int q = 0; q < 8; q++)
+                out[(size_t)(c / 4 + q) * WIDTH] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
         }
     }
     tc_fence_before();
     __syncthreads();
-    if ((EPI == EPI_LAST || EPI == EPI_BACK) && !abort_flag) {
-        for (int n = threadIdx.x; n < WIDTH; n += 128) {
-            g.db_partial[(size_t)blockIdx.x * WIDTH + n] = part_a[0][n] + part_a[1][n] + part_a[2][n] + part_a[3][n];
-            if (EPI == EPI_LAST)
-                g.dw5_partial[(size_t)blockIdx.x * WIDTH + n] = part_b[0][n] + part_b[1][n] + part_b[2][n] + part_b[3][n];
-        }
-        if (EPI == EPI_LAST && threadIdx.x < 2)
-            g.scalar_partial[2 * blockIdx.x + threadIdx.x] =
-                scal[0][threadIdx.x] + scal[1][threadIdx.x] + scal[2][threadIdx.x] + scal[3][threadIdx.x];
-    }
     tc_fence_after();
-    if (warp == 0) tmem_dealloc(tmem, COLS);
-}
-
-// ---- inputs into images ------------------------------------------------------------------------
-
-// x [batch][inputs] FP32 -> X as an A image (K = 64, zero padded) and X^T as a B image of 64 rows
-// (K = batch); one thread per (point, 8 features)
-__global__ void inputs_kernel(const float *x, uint32_t inputs, uint32_t batch, uint8_t *x_img, uint8_t *xt_img) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= batch * (IN / 8)) return;
-    const uint32_t m = t / (IN / 8), k0 = 8 * (t % (IN / 8));
-    uint32_t p[4];
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const uint32_t k = k0 + 2 * e;
-        const float lo = k < inputs ? x[(size_t)m * inputs + k] : 0.0f;
-        const float hi = k + 1 < inputs ? x[(size_t)m * inputs + k + 1] : 0.0f;
-        p[e] = pack_bf16(lo, hi);
-    }
-    *reinterpret_cast<uint4 *>(x_img + a_img(m, k0, 1)) = make_uint4(p[0], p[1], p[2], p[3]);
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const uint16_t bits = (uint16_t)(j & 1 ? p[j / 2] >> 16 : p[j / 2] & 0xffff);
-        *reinterpret_cast<uint16_t *>(xt_img + b_img(k0 + j, m, IN)) = bits;
-    }
+    if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
 // ---- parameters into weight images -----------------------------------------------------------
@@ -401,59 +544,145 @@ __global__ void images_kernel(const float *params, uint8_t *wimg, uint8_t *wtimg
 }
 
 // ---- gradients and Adam ----------------------------------------------------------------------------
+//
+// One launch sums the partials (each sum in a fixed order: the result does not depend on the launch),
+// and writes the gradient, or takes the Adam step with the weights' BF16 images: blocks 0 .. 207 a
+// piece of 16 rows x 64 columns of a layer's weights each, then 40 blocks of 32 bias or output weights
+// (eight segments of the tiles' sums side by side) and one of the scalars. The partials come by
+// (column / 4, row), the parameters, moments and images by rows, the transposed image by columns: a
+// piece turns between them in shared memory, so that every access is of whole sectors.
 
-struct GradArgs {
-    const float *dw[4];   // partials [splits][256][fan_in]
-    uint32_t splits;
-    const float *db[4];   // [blocks][256]
-    uint32_t blocks;
-    const float *dw5;     // [blocks][256]
-    const float *scalars; // [blocks][2]
-    float *grad;          // param order
+enum UpdateMode { UP_GRADIENT, UP_TRAIN, UP_APPLY };
+constexpr uint32_t UP_W = WIDTH / 16 * (1 + 3 * 4), UP_COLS = 5 * WIDTH / 32, UP_BLOCKS = UP_W + UP_COLS + 1;
+
+struct UpdateArgs {
+    const float *dw[4];   // [part][column / 4][row][4]
+    const float *db[4];   // [tile][256]
+    const float *dw5;     // [tile][256]
+    const float *scalars; // [tile][2]
+    uint32_t tiles;
+    float *grad;          // UP_GRADIENT: written; UP_APPLY: read (param order)
     float *loss;          // one float (set), or null
     float *loss_sum;      // one float (added), or null
+    float *params, *m1, *m2;
+    uint8_t *wimg, *wtimg;
+    float lr, c1, c2;
+    uint32_t inputs;
 };
 
-// one thread per parameter: the sum of its partials (in a fixed order: the result does not depend
-// on the launch)
-__global__ void grad_kernel(GradArgs a) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= P_COUNT) return;
-    float s = 0.0f;
-    if (t < P_B1) {
-        for (uint32_t k = 0; k < a.splits; k++) s += a.dw[0][(size_t)k * WIDTH * IN + t];
-    } else if (t >= P_W2 && t < P_B4 && (t - P_W2) % (WIDTH * WIDTH + WIDTH) < WIDTH * WIDTH) {
-        const uint32_t l = (uint32_t)((t - P_W2) / (WIDTH * WIDTH + WIDTH)), e = (uint32_t)((t - P_W2) % (WIDTH * WIDTH + WIDTH));
-        for (uint32_t k = 0; k < a.splits; k++) s += a.dw[l + 1][(size_t)k * WIDTH * WIDTH + e];
-    } else if (t < P_W5) {
-        // a bias of layers 1..4 (they follow their layer's weights)
-        const uint32_t layer = t < P_W2 ? 0 : t < P_W3 ? 1 : t < P_W4 ? 2 : 3;
-        const uint32_t n = (uint32_t)(t - (layer == 0 ? P_B1 : layer == 1 ? P_B2 : layer == 2 ? P_B3 : P_B4));
-        for (uint32_t k = 0; k < a.blocks; k++) s += a.db[layer][(size_t)k * WIDTH + n];
-    } else if (t < P_B5) {
-        for (uint32_t k = 0; k < a.blocks; k++) s += a.dw5[(size_t)k * WIDTH + (t - P_W5)];
-    } else {
-        float l = 0.0f;
-        for (uint32_t k = 0; k < a.blocks; k++) {
-            s += a.scalars[2 * k];
-            l += a.scalars[2 * k + 1];
-        }
-        if (a.loss) *a.loss = l;
-        if (a.loss_sum) *a.loss_sum += l;
-    }
-    a.grad[t] = s;
+// the Adam step of one value w with moments a and b on its gradient
+__device__ __forceinline__ void adam_value(const UpdateArgs &u, float &w, float &a, float &b, float g) {
+    a = 0.9f * a + 0.1f * g;
+    b = 0.999f * b + 0.001f * g * g;
+    w -= u.lr * (a * u.c1) / (sqrtf(b * u.c2) + 1e-8f);
 }
 
-__global__ void adam_kernel(float *params, float *m1, float *m2, const float *grad, float lr, float c1, float c2,
-                            uint32_t inputs) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= P_COUNT) return;
-    if (t < P_B1 && (t % IN) >= inputs) return;  // the padding columns of W1 stay zero
-    const float g = grad[t];
-    const float a = 0.9f * m1[t] + 0.1f * g, b = 0.999f * m2[t] + 0.001f * g * g;
-    m1[t] = a;
-    m2[t] = b;
-    params[t] -= lr * (a * c1) / (sqrtf(b * c2) + 1e-8f);
+template <int MODE> __device__ __forceinline__ void finish(const UpdateArgs &u, size_t t, float g) {
+    if (MODE == UP_GRADIENT) u.grad[t] = g;
+    else adam_value(u, u.params[t], u.m1[t], u.m2[t], MODE == UP_APPLY ? u.grad[t] : g);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(256) update_kernel(UpdateArgs u) {
+    __shared__ float red[8][33];
+    if (blockIdx.x < UP_W) {
+        __shared__ float4 piece[16][17];  // [row][column / 4]
+        const int layer = blockIdx.x < WIDTH / 16 ? 0 : 1 + (int)((blockIdx.x - WIDTH / 16) / (WIDTH / 16 * 4));
+        const uint32_t n = layer ? (blockIdx.x - WIDTH / 16) % (WIDTH / 16 * 4) : 4 * blockIdx.x;
+        const uint32_t row0 = 16 * (n / 4), first4 = 16 * (n % 4), fan = layer ? WIDTH : IN;
+        const uint32_t x = threadIdx.x & 15, y = threadIdx.x >> 4;
+        // by rows: this thread's row and columns
+        const uint32_t o = row0 + y, c4 = first4 + x;
+        const size_t t = (layer == 0 ? P_W1 : layer == 1 ? P_W2 : layer == 2 ? P_W3 : P_W4) + (size_t)o * fan + 4 * c4;
+        float4 w, a, b;
+        if (MODE != UP_GRADIENT) {  // (the network's own arrays: aligned)
+            w = *reinterpret_cast<const float4 *>(u.params + t);
+            a = *reinterpret_cast<const float4 *>(u.m1 + t);
+            b = *reinterpret_cast<const float4 *>(u.m2 + t);
+        }
+        float4 g;
+        if (MODE != UP_APPLY) {
+            const float4 *p = reinterpret_cast<const float4 *>(u.dw[layer]) + (size_t)(first4 + y) * WIDTH + row0 + x;
+            const uint32_t parts = dw_parts(layer, u.tiles);
+            g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 11
+            for (uint32_t k = 0; k < parts; k++) {
+                const float4 v = p[(size_t)k * fan / 4 * WIDTH];
+                g.x += v.x;
+                g.y += v.y;
+                g.z += v.z;
+                g.w += v.w;
+            }
+            piece[x][y] = g;
+            __syncthreads();
+            g = piece[y][x];
+        } else {  // (the caller's array, of any alignment)
+            g = make_float4(u.grad[t], u.grad[t + 1], u.grad[t + 2], u.grad[t + 3]);
+        }
+        if constexpr (MODE == UP_GRADIENT) {
+            u.grad[t] = g.x;
+            u.grad[t + 1] = g.y;
+            u.grad[t + 2] = g.z;
+            u.grad[t + 3] = g.w;
+        } else {
+            float *wv = &w.x, *av = &a.x, *bv = &b.x;
+            const float *gv = &g.x;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (layer > 0 || 4 * c4 + j < u.inputs) adam_value(u, wv[j], av[j], bv[j], gv[j]);  // (W1's padding columns stay zero)
+            *reinterpret_cast<float4 *>(u.params + t) = w;
+            *reinterpret_cast<float4 *>(u.m1 + t) = a;
+            *reinterpret_cast<float4 *>(u.m2 + t) = b;
+            *reinterpret_cast<uint2 *>(u.wimg + wimg_at(layer) + b_img(o, 4 * c4, WIDTH)) =
+                make_uint2(pack_bf16(w.x, w.y), pack_bf16(w.z, w.w));
+            if (layer > 0) {
+                __syncthreads();
+                piece[y][x] = w;
+                __syncthreads();
+                // by columns: eight rows of one column
+                if (threadIdx.x < 128) {
+                    const uint32_t c = threadIdx.x >> 1, r0 = 8 * (threadIdx.x & 1);
+                    const float *col = &piece[0][c / 4].x + c % 4;
+                    uint32_t q[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) q[j] = pack_bf16(col[(r0 + 2 * j) * 17 * 4], col[(r0 + 2 * j + 1) * 17 * 4]);
+                    *reinterpret_cast<uint4 *>(u.wtimg + (size_t)(layer - 1) * 4 * 256 * 128 + b_img(4 * first4 + c, row0 + r0, WIDTH)) =
+                        make_uint4(q[0], q[1], q[2], q[3]);
+                }
+            }
+        }
+    } else if (blockIdx.x < UP_W + UP_COLS) {
+        const uint32_t n = 32 * (blockIdx.x - UP_W) + (threadIdx.x & 31), layer = n / WIDTH, seg = threadIdx.x >> 5;
+        const float *src = (layer < 4 ? u.db[layer] : u.dw5) + n % WIDTH;
+        float s = 0.0f;
+        if (MODE != UP_APPLY) {
+#pragma unroll 8
+            for (uint32_t k = seg; k < u.tiles; k += 8) s += src[(size_t)k * WIDTH];
+            red[seg][threadIdx.x & 31] = s;
+            __syncthreads();
+            s = 0.0f;
+            for (int k = 0; k < 8; k++) s += red[k][threadIdx.x & 31];
+        }
+        if (seg == 0) finish<MODE>(u, (layer < 4 ? bias_at((int)layer) : P_W5) + n % WIDTH, s);
+    } else {
+        // the sum of dout (b5's gradient) and the loss: 128 strided sums each, then in order
+        __shared__ float sums[2][128];
+        const uint32_t which = threadIdx.x & 1, k0 = threadIdx.x >> 1;
+        float s = 0.0f;
+        if (MODE != UP_APPLY)
+            for (uint32_t k = k0; k < u.tiles; k += 128) s += u.scalars[2 * k + which];
+        sums[which][k0] = s;
+        __syncthreads();
+        if (threadIdx.x < 2) {
+            s = 0.0f;
+            for (int k = 0; k < 128; k++) s += sums[threadIdx.x][k];
+            if (threadIdx.x == 0) finish<MODE>(u, P_B5, s);
+            else if (MODE != UP_APPLY) {
+                if (u.loss) *u.loss = s;
+                if (u.loss_sum) *u.loss_sum += s;
+            }
+        }
+    }
 }
 
 // ---- fused inference ------------------------------------------------------------------------------
@@ -543,14 +772,6 @@ __device__ __forceinline__ void fwd_activate(const uint32_t (&z)[4][16], const f
     const float4 *b4 = reinterpret_cast<const float4 *>(bias);
 #pragma unroll
     for (int q = 0; q < 16; q++) fwd_activate4(&z[q / 4][4 * (q % 4)], b4[q], ph[2 * q], ph[2 * q + 1]);
-}
-
-// row r of one A tile from 32 packed pairs
-__device__ __forceinline__ void fwd_store_row(uint8_t *tile, uint32_t r, const uint32_t (&ph)[32]) {
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-        *reinterpret_cast<uint4 *>(tile + sw128_offset(r, 8 * q)) =
-            make_uint4(ph[4 * q], ph[4 * q + 1], ph[4 * q + 2], ph[4 * q + 3]);
 }
 
 template <int MODE>
@@ -755,7 +976,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) forward_kernel(ForwardArgs g) 
                 // (the second half's products have read the activations when they are done)
                 got = __all_sync(0xffffffffu, mbar_wait(&acc_ready[t][1], accs & 1, WAIT_CYCLES));
                 if (!got) break;
-                fwd_store_row(mine + c * TILE_A, r, ph);
+                store_row(mine + c * TILE_A, r, ph);
                 fence_async_shared();
                 tc_fence_before();
                 mbar_arrive(&act_ready[t][0]);
@@ -764,7 +985,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) forward_kernel(ForwardArgs g) 
                 if (!(got = take_turn())) break;
                 fwd_activate(z, bias + 128, ph);
                 pass_turn();
-                fwd_store_row(mine + (2 + c) * TILE_A, r, ph);
+                store_row(mine + (2 + c) * TILE_A, r, ph);
                 fence_async_shared();
                 tc_fence_before();
                 mbar_arrive(&act_ready[t][1]);
@@ -860,21 +1081,6 @@ bool failed(cudaError_t e, const char *step) {
     return true;
 }
 
-template <int N, int EPI>
-bool launch_gemm(const GemmArgs &g, uint32_t m_tiles, uint32_t splits, cudaStream_t s) {
-    static bool configured = false;
-    if (!configured) {
-        if (failed(cudaFuncSetAttribute(gemm_kernel<N, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        GemmShape<N>::SMEM),
-                   "product kernel attributes"))
-            return false;
-        configured = true;
-    }
-    gemm_kernel<N, EPI><<<dim3(m_tiles, splits), 128, GemmShape<N>::SMEM, s>>>(g);
-    g_last_launches++;
-    return !failed(cudaGetLastError(), "product kernel launch");
-}
-
 // tiles in flight per SM of the inference kernel: 2 or 1
 int g_forward_tiles = 2;
 
@@ -903,29 +1109,17 @@ bool launch_forward(ForwardArgs &g, cudaStream_t s) {
 struct pacuda_sg_net {
     uint32_t inputs = 0, max_batch = 0;
     uint64_t step = 0;
-    float *params = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr, *loss = nullptr;
+    float *params = nullptr, *m1 = nullptr, *m2 = nullptr;
     uint8_t *wimg = nullptr, *wtimg = nullptr;
     // workspace for a batch
-    uint8_t *x_img = nullptr, *xt_img = nullptr, *h_img[3] = {}, *ht_img[3] = {}, *dz_img[2] = {}, *dzt_img = nullptr;
-    __nv_bfloat16 *z[3] = {};
+    uint8_t *x_img = nullptr, *h_img[3] = {}, *dz_img[4] = {};
+    uint4 *z[3] = {};
     float *dw_part[4] = {}, *db_part[4] = {}, *dw5_part = nullptr, *scal_part = nullptr;
     int *error = nullptr;
-    std::vector<void *> owned;
+    void *slab = nullptr;  // one allocation for all of them
 };
 
 namespace {
-
-template <class T>
-bool dalloc(pacuda_sg_net *n, T **p, size_t bytes) {
-    void *q = nullptr;
-    if (failed(cudaMalloc(&q, bytes ? bytes : 16), "allocation")) return false;
-    n->owned.push_back(q);
-    *p = (T *)q;
-    return true;
-}
-
-// splits of the batch for the weight gradients: 4 tiles of K (256 points) per block when they divide
-uint32_t split_tiles(uint32_t batch) { return (batch / 64) % 4 == 0 ? 4 : 2; }
 
 int refresh_images(pacuda_sg_net *n, cudaStream_t s) {
     const uint32_t count = WIDTH * IN + 3 * WIDTH * WIDTH;
@@ -950,7 +1144,7 @@ extern "C" int pacuda_sg_set_inference_blocks(uint32_t blocks) {
 
 extern "C" void pacuda_sg_destroy(pacuda_sg_net *n) {
     if (!n) return;
-    for (void *p : n->owned) cudaFree(p);
+    cudaFree(n->slab);
     delete n;
 }
 
@@ -963,22 +1157,34 @@ extern "C" pacuda_sg_net *pacuda_sg_create(uint32_t inputs, uint32_t max_batch, 
     pacuda_sg_net *n = new pacuda_sg_net;
     n->inputs = inputs;
     n->max_batch = max_batch;
-    const size_t B = max_batch, blocks = B / 128, splits = B / 64 / 2;
-    bool ok = dalloc(n, &n->params, P_COUNT * 4) && dalloc(n, &n->m1, P_COUNT * 4) && dalloc(n, &n->m2, P_COUNT * 4) &&
-              dalloc(n, &n->grad, P_COUNT * 4) && dalloc(n, &n->loss, 16) && dalloc(n, &n->error, 16) &&
-              dalloc(n, &n->wimg, WIMG_BYTES) && dalloc(n, &n->wtimg, 3 * 4 * 256 * 128) &&
-              dalloc(n, &n->x_img, B * IN * 2) && dalloc(n, &n->xt_img, B * IN * 2) && dalloc(n, &n->dzt_img, B * WIDTH * 2) &&
-              dalloc(n, &n->dw5_part, blocks * WIDTH * 4) && dalloc(n, &n->scal_part, blocks * 2 * 4);
-    for (int l = 0; ok && l < 3; l++)
-        ok = dalloc(n, &n->h_img[l], B * WIDTH * 2) && dalloc(n, &n->ht_img[l], B * WIDTH * 2) &&
-             dalloc(n, &n->z[l], B * WIDTH * 2);
-    for (int l = 0; ok && l < 2; l++) ok = dalloc(n, &n->dz_img[l], B * WIDTH * 2);
-    for (int l = 0; ok && l < 4; l++)
-        ok = dalloc(n, &n->dw_part[l], splits * WIDTH * (l == 0 ? IN : WIDTH) * 4) && dalloc(n, &n->db_part[l], blocks * WIDTH * 4);
-    if (!ok) {
+    const size_t B = max_batch, tiles = B / 128;
+    std::vector<std::pair<void **, size_t>> arrays;
+    size_t total = 0;
+    auto array = [&](auto **p, size_t bytes) {
+        arrays.push_back({(void **)p, total});
+        total += (bytes + 255) / 256 * 256;
+    };
+    for (float **p : {&n->params, &n->m1, &n->m2}) array(p, P_COUNT * 4);
+    array(&n->error, 16);
+    array(&n->wimg, WIMG_BYTES);
+    array(&n->wtimg, 3 * 4 * 256 * 128);
+    array(&n->x_img, B * IN * 2);
+    array(&n->dw5_part, tiles * WIDTH * 4);
+    array(&n->scal_part, tiles * 2 * 4);
+    for (int l = 0; l < 3; l++) {
+        array(&n->h_img[l], B * WIDTH * 2);
+        array(&n->z[l], B * WIDTH * 2);
+    }
+    for (int l = 0; l < 4; l++) {
+        array(&n->dz_img[l], B * WIDTH * 2);
+        array(&n->db_part[l], tiles * WIDTH * 4);
+        array(&n->dw_part[l], (size_t)dw_parts(l, (uint32_t)tiles) * WIDTH * (l == 0 ? IN : WIDTH) * 4);
+    }
+    if (failed(cudaMalloc(&n->slab, total), "allocation")) {
         pacuda_sg_destroy(n);
         return nullptr;
     }
+    for (auto &a : arrays) *a.first = (uint8_t *)n->slab + a.second;
     // weights uniform in +-sqrt(6 / fan_in) from a splitmix64 stream, biases zero
     std::vector<float> p(P_COUNT, 0.0f);
     uint64_t state = seed;
@@ -1025,103 +1231,84 @@ extern "C" int pacuda_sg_get_params(const pacuda_sg_net *n, float *params) {
 
 namespace {
 
-// the forward and backward products of one batch and the reduction of their partials into the
-// gradient (param order) and the loss
-int gradients(pacuda_sg_net *n, const float *x, const float *y, uint32_t batch, float *grad, float *loss,
-              float *loss_sum, cudaStream_t s) {
-    if (!n || !x || !y || !grad || batch == 0 || batch % 128 || batch > n->max_batch) {
+template <class F> bool allow_shared(F *kernel, uint32_t bytes, const char *what) {
+    return !failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), what);
+}
+
+// the forward and backward chain and the weight gradients' partials of one batch; `u` gets what the
+// update reads of them
+int products(pacuda_sg_net *n, const float *x, const float *y, uint32_t batch, UpdateArgs &u, cudaStream_t s) {
+    if (!n || !x || !y || batch == 0 || batch % 128 || batch > n->max_batch) {
         fprintf(stderr, "%s: a batch of %u points (a multiple of 128, at most %u)\n", kTag, batch, n ? n->max_batch : 0);
         return ST_INVALID;
     }
-    const uint32_t blocks = batch / 128, st = split_tiles(batch), splits = batch / 64 / st, kt = batch / 64;
-    inputs_kernel<<<(batch * (IN / 8) + 255) / 256, 256, 0, s>>>(x, n->inputs, batch, n->x_img, n->xt_img);
-    g_last_launches++;
-    if (failed(cudaGetLastError(), "inputs")) return ST_DEVICE;
-    GemmArgs g;
-    memset(&g, 0, sizeof g);
-    g.batch = batch;
-    g.error = n->error;
-    g.inv_batch = 1.0f / (float)batch;
-    // forward, layers 1-3
+    static bool configured = false;
+    if (!configured) {
+        if (!allow_shared(chain_kernel, CH_SMEM, "chain attributes") || !allow_shared(dw_kernel, DW_SMEM, "weight gradient attributes"))
+            return ST_DEVICE;
+        configured = true;
+    }
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint32_t tiles = batch / 128;
+    ChainArgs c;
+    DwArgs d;
+    memset(&u, 0, sizeof u);
+    c.wimg = n->wimg;
+    c.wtimg = n->wtimg;
+    c.params = n->params;
+    c.x = x;
+    c.y = y;
+    c.inputs = n->inputs;
+    c.tiles = d.tiles = u.tiles = tiles;
+    c.inv_batch = 1.0f / (float)batch;
+    c.x_img = n->x_img;
+    d.x_img = n->x_img;
     for (int l = 0; l < 3; l++) {
-        g.a = l == 0 ? n->x_img : n->h_img[l - 1];
-        g.a_kt = g.k_tiles = l == 0 ? 1 : 4;
-        g.b = n->wimg + wimg_at(l);
-        g.bias = n->params + bias_at(l);
-        g.h_img = n->h_img[l];
-        g.ht_img = n->ht_img[l];
-        g.z = n->z[l];
-        if (!launch_gemm<256, EPI_HIDDEN>(g, blocks, 1, s)) return ST_DEVICE;
+        c.h_img[l] = n->h_img[l];
+        d.h_img[l] = n->h_img[l];
+        c.z[l] = n->z[l];
     }
-    // layer 4 and the output layer: dZ4
-    g.a = n->h_img[2];
-    g.a_kt = g.k_tiles = 4;
-    g.b = n->wimg + wimg_at(3);
-    g.bias = n->params + P_B4;
-    g.w5 = n->params + P_W5;
-    g.b5 = n->params + P_B5;
-    g.y = y;
-    g.dz_img = n->dz_img[0];
-    g.dzt_img = n->dzt_img;
-    g.db_partial = n->db_part[3];
-    g.dw5_partial = n->dw5_part;
-    g.scalar_partial = n->scal_part;
-    if (!launch_gemm<256, EPI_LAST>(g, blocks, 1, s)) return ST_DEVICE;
-    // backward: layer l = 4, 3, 2 (index 3, 2, 1): dW_l, then dZ_{l-1}
-    int cur = 0;
-    for (int l = 3; l >= 1; l--) {
-        GemmArgs w;
-        memset(&w, 0, sizeof w);
-        w.error = n->error;
-        w.a = n->dzt_img;
-        w.a_kt = kt;
-        w.k_tiles = st;
-        w.b = n->ht_img[l - 1];
-        w.partial = n->dw_part[l];
-        w.m_rows = WIDTH;
-        if (!launch_gemm<256, EPI_PARTIAL>(w, 2, splits, s)) return ST_DEVICE;
-        GemmArgs d;
-        memset(&d, 0, sizeof d);
-        d.error = n->error;
-        d.batch = batch;
-        d.a = n->dz_img[cur];
-        d.a_kt = d.k_tiles = 4;
-        d.b = n->wtimg + (size_t)(l - 1) * 4 * 256 * 128;
-        d.zprev = n->z[l - 1];
-        d.dz_img = n->dz_img[cur ^ 1];
-        d.dzt_img = n->dzt_img;
-        d.db_partial = n->db_part[l - 1];
-        if (!launch_gemm<256, EPI_BACK>(d, blocks, 1, s)) return ST_DEVICE;
-        cur ^= 1;
-    }
-    // dW1 = dZ1^T X
-    {
-        GemmArgs w;
-        memset(&w, 0, sizeof w);
-        w.error = n->error;
-        w.a = n->dzt_img;
-        w.a_kt = kt;
-        w.k_tiles = st;
-        w.b = n->xt_img;
-        w.partial = n->dw_part[0];
-        w.m_rows = WIDTH;
-        if (!launch_gemm<64, EPI_PARTIAL>(w, 2, splits, s)) return ST_DEVICE;
-    }
-    GradArgs a;
     for (int l = 0; l < 4; l++) {
-        a.dw[l] = n->dw_part[l];
-        a.db[l] = n->db_part[l];
+        c.dz_img[l] = n->dz_img[l];
+        d.dz_img[l] = n->dz_img[l];
+        c.db[l] = n->db_part[l];
+        u.db[l] = n->db_part[l];
+        d.partial[l] = n->dw_part[l];
+        u.dw[l] = n->dw_part[l];
     }
-    a.splits = splits;
-    a.blocks = blocks;
-    a.dw5 = n->dw5_part;
-    a.scalars = n->scal_part;
-    a.grad = grad;
-    a.loss = loss;
-    a.loss_sum = loss_sum;
-    grad_kernel<<<(unsigned)((P_COUNT + 255) / 256), 256, 0, s>>>(a);
+    c.dw5 = n->dw5_part;
+    u.dw5 = n->dw5_part;
+    c.scalars = n->scal_part;
+    u.scalars = n->scal_part;
+    c.error = d.error = n->error;
+    chain_kernel<<<tiles < (uint32_t)sms ? tiles : (uint32_t)sms, CH_THREADS, CH_SMEM, s>>>(c);
     g_last_launches++;
-    return failed(cudaGetLastError(), "gradient reduction") ? ST_DEVICE : ST_OK;
+    if (failed(cudaGetLastError(), "forward and backward")) return ST_DEVICE;
+    dw_kernel<<<6 * dw_parts(1, tiles) + 2 * dw_parts(0, tiles), 256, DW_SMEM, s>>>(d);
+    g_last_launches++;
+    return failed(cudaGetLastError(), "weight gradients") ? ST_DEVICE : ST_OK;
+}
+
+// the gradient of one batch into `grad` (UP_GRADIENT), the Adam step on it (UP_TRAIN), or on a given
+// gradient (UP_APPLY)
+template <int MODE> int update(pacuda_sg_net *n, UpdateArgs &u, float lr, cudaStream_t s) {
+    u.params = n->params;
+    u.m1 = n->m1;
+    u.m2 = n->m2;
+    u.wimg = n->wimg;
+    u.wtimg = n->wtimg;
+    u.inputs = n->inputs;
+    if (MODE != UP_GRADIENT) {
+        n->step++;
+        u.lr = lr;
+        u.c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)n->step)));
+        u.c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)n->step)));
+    }
+    update_kernel<MODE><<<UP_BLOCKS, 256, 0, s>>>(u);
+    g_last_launches++;
+    return failed(cudaGetLastError(), "update") ? ST_DEVICE : ST_OK;
 }
 
 }  // namespace
@@ -1129,37 +1316,32 @@ int gradients(pacuda_sg_net *n, const float *x, const float *y, uint32_t batch, 
 extern "C" int pacuda_sg_gradients(pacuda_sg_net *n, const float *x, const float *y, uint32_t batch, float *grad,
                                    float *loss, void *stream) {
     g_last_launches = 0;
-    return gradients(n, x, y, batch, grad, loss, nullptr, (cudaStream_t)stream);
+    if (!grad) return ST_INVALID;
+    UpdateArgs u;
+    int st = products(n, x, y, batch, u, (cudaStream_t)stream);
+    if (st != ST_OK) return st;
+    u.grad = grad;
+    u.loss = loss;
+    return update<UP_GRADIENT>(n, u, 0.0f, (cudaStream_t)stream);
 }
-
-namespace {
-
-// one Adam step on the gradient `grad` (param order, device) and the weight images
-int adam_step(pacuda_sg_net *n, const float *grad, float lr, cudaStream_t s) {
-    n->step++;
-    const float c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)n->step)));
-    const float c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)n->step)));
-    adam_kernel<<<(unsigned)((P_COUNT + 255) / 256), 256, 0, s>>>(n->params, n->m1, n->m2, grad, lr, c1, c2, n->inputs);
-    g_last_launches++;
-    if (failed(cudaGetLastError(), "adam")) return ST_DEVICE;
-    return refresh_images(n, s);
-}
-
-}  // namespace
 
 extern "C" int pacuda_sg_apply_gradients(pacuda_sg_net *n, const float *grad, float lr, void *stream) {
     g_last_launches = 0;
     if (!n || !grad) return ST_INVALID;
-    return adam_step(n, grad, lr, (cudaStream_t)stream);
+    UpdateArgs u;
+    memset(&u, 0, sizeof u);
+    u.grad = const_cast<float *>(grad);
+    return update<UP_APPLY>(n, u, lr, (cudaStream_t)stream);
 }
 
 extern "C" int pacuda_sg_train_step(pacuda_sg_net *n, const float *x, const float *y, uint32_t batch, float lr,
                                     float *loss_sum, void *stream) {
     g_last_launches = 0;
-    cudaStream_t s = (cudaStream_t)stream;
-    int st = gradients(n, x, y, batch, n ? n->grad : nullptr, nullptr, loss_sum, s);
+    UpdateArgs u;
+    int st = products(n, x, y, batch, u, (cudaStream_t)stream);
     if (st != ST_OK) return st;
-    return adam_step(n, n->grad, lr, s);
+    u.loss_sum = loss_sum;
+    return update<UP_TRAIN>(n, u, lr, (cudaStream_t)stream);
 }
 
 extern "C" int pacuda_sg_forward(const pacuda_sg_net *n, const float *x, uint32_t count, float *out, void *stream) {

@@ -61,6 +61,17 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  : "memory");
 }
 
+// `bytes` (a multiple of 16) of shared memory to 16-byte aligned global memory as one bulk group of this
+// thread; the writes to shared memory must be visible to the async proxy (fence_async_shared)
+__device__ __forceinline__ void bulk_store(void *dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// this thread's bulk stores have read their shared memory; and: are complete
+__device__ __forceinline__ void bulk_store_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // ---- fences --------------------------------------------------------------------------------------
 
 // generic-proxy writes to shared memory made visible to the tensor cores' reads
@@ -131,6 +142,19 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
     d |= (uint64_t)2 << 61;                           // 128-byte swizzle
     return d;
 }
+
+// The same image read with its roles exchanged (MN-major): rows are K, the 64 values of a row are M or
+// N. `addr`: the first tile at the first of the K rows (+2048 bytes per 16 rows); `group` bytes from
+// one tile (64 values of M or N) to the next.
+__device__ __forceinline__ uint64_t sw128_mn_desc(uint32_t addr, uint32_t group) {
+    uint64_t d = (uint64_t)((addr & 0x3FFFF) >> 4);
+    d |= (uint64_t)(group >> 4) << 16;                // leading byte offset: the next 64 values of M or N
+    d |= (uint64_t)(1024 >> 4) << 32;                 // stride byte offset: the next 8 rows of K
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+constexpr uint32_t IDESC_MN = 1u << 15 | 1u << 16;    // instruction descriptor: A and B MN-major
 
 // instruction descriptor of kind::f16: A and B BF16, D FP32, both K-major, M x N
 __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N) {
