@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
     typedef typename K::Den Den;
     typedef typename K::Amp Amp;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ unsigned long long next_item;
+    __shared__ unsigned long long next_item[2];  // by turns: this item and (AHEAD) the one after it
     // The block's shared memory from its address in a register: taken from the array's symbol, every
     // row computes that address again (6 of 190 instructions; gg>ggg 4096 points 146 -> 143 us,
     // qg>qgg 125 -> 130 M points/s). The C ABI's kernel has no register left for it.
@@ -632,10 +632,22 @@ __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
         block = (unsigned char *)__cvta_shared_to_generic(window);
     }
     const unsigned long long total = L.item_first[L.nplans];
-    while (true) {
-        if (threadIdx.x == 0) next_item = atomicAdd(L.counter, 1ull);
+    // The counter's answer comes from L2. Asked for an item ahead, it comes while the item's forms wait
+    // for memory: the df64 plans run one or two blocks per SM, whose other blocks do not cover that wait
+    // (65 537 points of the 3-jet mix: 6.93 -> 6.14 ms). In f64 four blocks cover it, and one more value
+    // that stays through the levels is spilled, to the little L1 that the instructions stream
+    // through (4096 points of gg>ggg: 143 -> 153 us).
+    constexpr bool AHEAD = !is_f64<R>::value;
+    if (AHEAD) {
+        if (threadIdx.x == 0) next_item[0] = atomicAdd(L.counter, 1ull);
         __syncthreads();
-        const unsigned long long item = next_item;
+    }
+    for (uint32_t turn = 0;; turn ^= AHEAD) {
+        if (!AHEAD) {
+            if (threadIdx.x == 0) next_item[0] = atomicAdd(L.counter, 1ull);
+            __syncthreads();
+        }
+        const unsigned long long item = next_item[turn];
         if (item >= total) break;
         uint32_t k = 0;
         while (item >= L.item_first[k + 1]) k++;
@@ -672,6 +684,8 @@ __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
         uint32_t plain = 0;
         while (true) {
             bool bad = false;
+            unsigned long long ahead = 0;
+            if (AHEAD && threadIdx.x == 0 && !plain) ahead = atomicAdd(L.counter, 1ull);
             if (active) {
                 const uint32_t count = L.count[k];
                 const size_t mine = (size_t)(item - L.item_first[k]) * np + pw;
@@ -713,6 +727,7 @@ __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
                     for (uint32_t t = tl; t < p.terms; t += lanes) v.put_term(t, konst<Amp>(0.0), konst<Amp>(0.0));
                 }
             }
+            if (AHEAD && threadIdx.x == 0 && !plain) next_item[turn ^ 1] = ahead;
             __syncthreads();  // the forms and live-in values are in
             // batches of one point per block (six-leg plans, gg>ggg) and of eight (the 5-leg quark
             // plans at two blocks per SM) run a copy of the levels with that count built in; in the C
