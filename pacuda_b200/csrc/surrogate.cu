@@ -20,6 +20,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -110,7 +111,7 @@ __device__ __forceinline__ void flag_error(int *error, int code, volatile int *a
 // bounds it: a product is 2 048 cycles of the tensor pipe, an epilogue as many of the MUFU (a tanh
 // per value). As seven launches, each with its operands read from and written to global memory, its
 // transposed copies stored in 2-byte pieces and four epilogue warps, this part took 127 us of a
-// step's 206; here 35 of 69 (68 thousand cycles per tile: 3 to 4 for each product with its operand's
+// step's 206; here 35 of 71 (68 thousand cycles per tile: 3 to 4 for each product with its operand's
 // hand-over, 4.5 to 5 for an epilogue, 11 for the output layer's).
 
 constexpr int CH_EPI = 512, CH_THREADS = CH_EPI + 64, CH_STAGES = 4;
@@ -130,6 +131,16 @@ struct ChainArgs {
     float *scalars;          // [tile][2]: sum dout, sum (out - y)^2
     int *error;
 };
+
+// A training step's three kernels are launched ahead of their turn (launch_early): a block sets up
+// its barriers and tensor memory, and the update its parameters, while the kernel before runs out.
+// grid_wait: until that kernel is complete and its writes are seen; everything that an earlier kernel
+// wrote, or still reads, is touched behind it. grid_trigger: the next kernel's blocks may be placed. Every
+// block triggers behind its own wait, so a placed kernel knows that the one before the one it waits
+// for is complete (what the update loads ahead was written by the step before).
+// 16 steps of 16 384 points: 1264 -> 1135 us (8 us of a step's 79 were the three kernels' ends and starts).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // row r of one A tile from 32 packed pairs
 __device__ __forceinline__ void store_row(uint8_t *tile, uint32_t r, const uint32_t (&ph)[32]) {
@@ -163,9 +174,11 @@ __global__ void __launch_bounds__(CH_THREADS, 1) chain_kernel(ChainArgs g) {
         abort_flag = 0;
         fence_mbar_init();
     }
+    if (warp == 0) tmem_alloc(&tmem_base, 256);
+    grid_wait();
+    grid_trigger();
     for (int i = threadIdx.x; i < 4 * WIDTH; i += CH_THREADS) bias[i / WIDTH][i % WIDTH] = g.params[bias_at(i / WIDTH) + i % WIDTH];
     for (int i = threadIdx.x; i <= WIDTH; i += CH_THREADS) w5[i] = g.params[P_W5 + i];  // (then b5)
-    if (warp == 0) tmem_alloc(&tmem_base, 256);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -446,6 +459,8 @@ __global__ void __launch_bounds__(256, 1) dw_kernel(DwArgs g) {
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(&tmem_base, 256);
+    grid_wait();
+    grid_trigger();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -600,6 +615,8 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs u) {
             a = *reinterpret_cast<const float4 *>(u.m1 + t);
             b = *reinterpret_cast<const float4 *>(u.m2 + t);
         }
+        grid_wait();
+        grid_trigger();
         float4 g;
         if (MODE != UP_APPLY) {
             const float4 *p = reinterpret_cast<const float4 *>(u.dw[layer]) + (size_t)(first4 + y) * WIDTH + row0 + x;
@@ -655,6 +672,8 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs u) {
         const uint32_t n = 32 * (blockIdx.x - UP_W) + (threadIdx.x & 31), layer = n / WIDTH, seg = threadIdx.x >> 5;
         const float *src = (layer < 4 ? u.db[layer] : u.dw5) + n % WIDTH;
         float s = 0.0f;
+        grid_wait();
+        grid_trigger();
         if (MODE != UP_APPLY) {
 #pragma unroll 8
             for (uint32_t k = seg; k < u.tiles; k += 8) s += src[(size_t)k * WIDTH];
@@ -669,6 +688,8 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs u) {
         __shared__ float sums[2][128];
         const uint32_t which = threadIdx.x & 1, k0 = threadIdx.x >> 1;
         float s = 0.0f;
+        grid_wait();
+        grid_trigger();
         if (MODE != UP_APPLY)
             for (uint32_t k = k0; k < u.tiles; k += 128) s += u.scalars[2 * k + which];
         sums[which][k0] = s;
@@ -1235,6 +1256,25 @@ template <class F> bool allow_shared(F *kernel, uint32_t bytes, const char *what
     return !failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), what);
 }
 
+// launches `kernel` so that it may be set up while the stream's kernel before it ends (grid_wait)
+template <class A>
+bool launch_early(void (*kernel)(A), uint32_t blocks, uint32_t threads, uint32_t shared, cudaStream_t s, const A &args, const char *what) {
+    cudaLaunchAttribute early;
+    memset(&early, 0, sizeof early);
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c;
+    memset(&c, 0, sizeof c);
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = shared;
+    c.stream = s;
+    c.attrs = &early;
+    c.numAttrs = 1;
+    g_last_launches++;
+    return !failed(cudaLaunchKernelEx(&c, kernel, args), what);
+}
+
 // the forward and backward chain and the weight gradients' partials of one batch; `u` gets what the
 // update reads of them
 int products(pacuda_sg_net *n, const float *x, const float *y, uint32_t batch, UpdateArgs &u, cudaStream_t s) {
@@ -1283,12 +1323,10 @@ int products(pacuda_sg_net *n, const float *x, const float *y, uint32_t batch, U
     c.scalars = n->scal_part;
     u.scalars = n->scal_part;
     c.error = d.error = n->error;
-    chain_kernel<<<tiles < (uint32_t)sms ? tiles : (uint32_t)sms, CH_THREADS, CH_SMEM, s>>>(c);
-    g_last_launches++;
-    if (failed(cudaGetLastError(), "forward and backward")) return ST_DEVICE;
-    dw_kernel<<<6 * dw_parts(1, tiles) + 2 * dw_parts(0, tiles), 256, DW_SMEM, s>>>(d);
-    g_last_launches++;
-    return failed(cudaGetLastError(), "weight gradients") ? ST_DEVICE : ST_OK;
+    return launch_early(chain_kernel, std::min(tiles, (uint32_t)sms), CH_THREADS, CH_SMEM, s, c, "forward and backward") &&
+                   launch_early(dw_kernel, 6 * dw_parts(1, tiles) + 2 * dw_parts(0, tiles), 256, DW_SMEM, s, d, "weight gradients")
+               ? ST_OK
+               : ST_DEVICE;
 }
 
 // the gradient of one batch into `grad` (UP_GRADIENT), the Adam step on it (UP_TRAIN), or on a given
@@ -1306,6 +1344,8 @@ template <int MODE> int update(pacuda_sg_net *n, UpdateArgs &u, float lr, cudaSt
         u.c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)n->step)));
         u.c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)n->step)));
     }
+    if (MODE != UP_APPLY) return launch_early(update_kernel<MODE>, UP_BLOCKS, 256, 0, s, u, "update") ? ST_OK : ST_DEVICE;
+    // (after another kernel than this step's the parameters that it loads before it waits may not be in)
     update_kernel<MODE><<<UP_BLOCKS, 256, 0, s>>>(u);
     g_last_launches++;
     return failed(cudaGetLastError(), "update") ? ST_DEVICE : ST_OK;
