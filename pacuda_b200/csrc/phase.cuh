@@ -216,18 +216,18 @@ template <int L> __device__ __forceinline__ bool passes(const double (&p)[L][4],
     return true;
 }
 
-// ---- a first look in f32: candidates that certainly fail the cuts ----------------------------
+// ---- a first look in f32: candidates that certainly fail or pass the cuts ----------------------
 // The f64 map above defines every candidate's point, and the cuts on it decide the list. Most
-// candidates fail by a wide margin (a soft or collinear parton), so the listing first maps each
-// one in f32, written to stay accurate where the f64 form cancels: 1 - sigma, cos(theta) and
+// candidates fail or pass by a wide margin (a soft or collinear parton, three hard ones), so the
+// listing first maps each one in f32, written to stay accurate where the f64 form cancels: 1 - sigma, cos(theta) and
 // sin(theta) from one exponential each, and a boost by velocity |q| / E_q of a frame of mass m
 // with gamma - 1 = |q|^2 / (m (E_q + m)) and gamma beta = |q| / m instead of 1 / sqrt(1 - beta^2).
 // Its uniforms are the same stream's states read to 24 bits, its exponentials and angles the
 // hardware approximations (relative errors near 2^-21). Every final-state component it gives then
 // differs from the f64 map's by about 5e-7 sqrt(s) at most (the 24-bit uniforms dominate; a float32
 // restatement of these formulas on 4e5 candidates of each map stays below that against the f64
-// map), 40 times less than the margin: a candidate is dropped here only when it fails a cut by more
-// than PHASE32_DELTA = 2e-5 sqrt(s) per component allows (pT by 2 delta, |pz| - pT sinh(eta_max)
+// map), 40 times less than the margin: a candidate is dropped here only when it fails a cut, and
+// listed only when it passes every cut, by more than PHASE32_DELTA = 2e-5 sqrt(s) per component allows (pT by 2 delta, |pz| - pT sinh(eta_max)
 // by (1 + 1.5 sinh(eta_max)) delta, Delta R by the propagated bounds on eta and phi). Every other
 // candidate goes through the f64 map and cuts, so the list is the f64 decision's.
 constexpr float PHASE32_DELTA = 2e-5f;
@@ -331,20 +331,27 @@ __device__ __forceinline__ void final32(const float (&u)[Space<4>::NUMBERS], dou
     boost32(mq, eq, e1, w, en4, q4, p[3]);
 }
 
-// whether the candidate whose f32 partons are p certainly fails the cuts (see above)
+// What the f32 partons p say of a candidate's cuts (see above). The margins hold both ways: a value
+// beyond the cut by more than its error is beyond it in f64, on either side. (Comparisons are written
+// so that a NaN is not sure of anything; past 1e18 the squares of f32 overflow.)
+enum Look : uint32_t { LOOK_FAILS, LOOK_PASSES, LOOK_UNSURE };
 template <int F>
-__device__ __forceinline__ bool surely_fails32(const float (&p)[F][3], double sqrt_s, const Cuts &c) {
-    const float d = PHASE32_DELTA * (float)sqrt_s, sh = sinhf((float)c.eta_max);
+__device__ __forceinline__ Look look32(const float (&p)[F][3], double sqrt_s, const Cuts &c) {
+    const float d = PHASE32_DELTA * (float)sqrt_s, sh = sinhf((float)c.eta_max), dz = d * (1.0f + 1.5f * sh);
+    bool sure = true;
     float pt[F];
     for (int i = 0; i < F; i++) {
         pt[i] = sqrtf(p[i][0] * p[i][0] + p[i][1] * p[i][1]);
-        if (pt[i] < (float)c.pt_min - 2.0f * d) return true;
-        if (fabsf(p[i][2]) - pt[i] * sh > d * (1.0f + 1.5f * sh)) return true;
+        const float over = fabsf(p[i][2]) - pt[i] * sh;
+        if (pt[i] < (float)c.pt_min - 2.0f * d) return LOOK_FAILS;
+        if (over > dz) return LOOK_FAILS;
+        // (the f64 cut compares pT^2 with pt_min^2: a negative pt_min cuts like its size)
+        sure = sure && pt[i] > fabsf((float)c.pt_min) + 2.0f * d && -over > dz;
     }
     float eta[F], phi[F], err[F];
     for (int i = 0; i < F; i++) {
         const float low = pt[i] - 2.0f * d;
-        if (!(low > 0.0f)) return false;
+        if (!(low > 0.0f) || !(pt[i] < 1e18f)) return LOOK_UNSURE;
         const float z = p[i][2] / pt[i];
         eta[i] = copysignf(__logf(fabsf(z) + sqrtf(z * z + 1.0f)), z);
         phi[i] = atan2f(p[i][1], p[i][0]);
@@ -355,10 +362,11 @@ __device__ __forceinline__ bool surely_fails32(const float (&p)[F][3], double sq
         for (int j = i + 1; j < F; j++) {
             float dp = fabsf(phi[i] - phi[j]);
             if (dp > pi) dp = 2.0f * pi - dp;
-            const float de = eta[i] - eta[j];
-            if (sqrtf(de * de + dp * dp) + err[i] + err[j] + 1e-5f < (float)c.dr_min) return true;
+            const float de = eta[i] - eta[j], r = sqrtf(de * de + dp * dp), e = err[i] + err[j] + 1e-5f;
+            if (r + e < (float)c.dr_min) return LOOK_FAILS;
+            sure = sure && r - e > fabsf((float)c.dr_min);
         }
-    return false;
+    return sure ? LOOK_PASSES : LOOK_UNSURE;
 }
 
 }  // namespace phase
