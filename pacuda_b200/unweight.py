@@ -163,6 +163,9 @@ class Pipeline:
         self.counters = torch.zeros(2 * nf, dtype=torch.int64, device="cuda")
         plans, moms, outs = self._parts([f.momenta[: 4 * f.legs * 1024] for f in self.fams], [1024] * nf)
         self.batch = B.Batch(plans, moms, outs)
+        # until tune() has timed the plans' choices: by their points' size (a two-stage step of 2^22
+        # candidates, some 20 000 of them evaluated, 1.87 ms at one block per SM, 1.74 so)
+        self.batch.blocks_per_sm = 0
 
     def _parts(self, moms, counts):
         """Every family's plans with their momenta and output buffers (the batch's order)."""
