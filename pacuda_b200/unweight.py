@@ -135,8 +135,8 @@ class Events:
 
     def compact(self):
         """(indices, weights) of the kept events (new tensors)."""
-        keep = self.keep_flags.bool()
-        return self.points[keep].clone(), self.all_weights[keep].clone()
+        at = self.keep_flags.nonzero().view(-1)  # (one wait for their number)
+        return self.points[at], self.all_weights[at]
 
 
 class Pipeline:
