@@ -103,16 +103,25 @@ __device__ __forceinline__ void flag_error(int *error, int code, volatile int *a
 // One block per 128 points at a time: seven products (four layers forward, three back) one after the
 // other, each on the operand that the epilogue before it left in shared memory. Warps 0-15 run the
 // epilogues: thread (quarter, lane, c) owns point r = 32 quarter + lane, tensor-memory lane r, and
-// the 64 columns of quarter c; warp 16 streams the weight images (32 KB chunks: a k tile of all 256
-// rows), warp 17 issues the products (M = 128, N = 256). Z stays with the thread that made it: it
-// goes to global memory and back in the order of the threads.
+// columns [32 c, 32 c + 32) of each half of 128 columns; warp 16 streams the weight images (32 KB
+// chunks: a k tile of all 256 rows), warp 17 issues the products (M = 128, N = 128 per half). Z
+// stays with the thread that made it: it goes to global memory and back in the order of the threads.
+//
+// The halves overlap a layer with the next one. A product's k tiles 0 and 1 (of both column halves)
+// need only the operand's first half, and go under the epilogue of its second half; k tiles 2 and 3
+// of the first column half follow, are committed, and the next epilogue starts on them while those
+// of the second column half run. Consecutive products use the two accumulators of 256 columns in
+// turn. The operand is replaced in place: the commit of a column half tracks every product issued
+// before it, which for the first are all those that read the operand's first half.
 //
 // At the training batch (16 384 points, 128 blocks) the chain of products and epilogues is what
 // bounds it: a product is 2 048 cycles of the tensor pipe, an epilogue as many of the MUFU (a tanh
 // per value). As seven launches, each with its operands read from and written to global memory, its
 // transposed copies stored in 2-byte pieces and four epilogue warps, this part took 127 us of a
-// step's 206; here 35 of 71 (68 thousand cycles per tile: 3 to 4 for each product with its operand's
-// hand-over, 4.5 to 5 for an epilogue, 11 for the output layer's).
+// step's 206. In one launch with whole layers one after the other: 68 thousand cycles per tile (35 us,
+// a step 70.5 us); with the overlapping halves, the columns' sums behind the hand-overs and Z asked
+// for ahead: 59 thousand (a step 65.5 us): a half's wait for its products 1.2 or 0.25 thousand
+// forward, 2.2 or 1.5 back (the columns' sums in it), its epilogue 2 to 2.9, the output layer's 11.
 
 constexpr int CH_EPI = 512, CH_THREADS = CH_EPI + 64, CH_STAGES = 4;
 constexpr uint32_t CH_CHUNK = 256 * 128;  // 32 KB
@@ -154,7 +163,7 @@ __device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, 5
 
 __global__ void __launch_bounds__(CH_THREADS, 1) chain_kernel(ChainArgs g) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full[CH_STAGES], empty[CH_STAGES], act_ready, acc_ready;
+    __shared__ uint64_t full[CH_STAGES], empty[CH_STAGES], act_ready[2], acc_ready[2];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
     __shared__ __align__(16) float bias[4][WIDTH], w5[WIDTH + 4];
@@ -169,12 +178,14 @@ __global__ void __launch_bounds__(CH_THREADS, 1) chain_kernel(ChainArgs g) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        mbar_init(&act_ready, 1);
-        mbar_init(&acc_ready, 1);
+        for (int h = 0; h < 2; h++) {
+            mbar_init(&act_ready[h], 1);
+            mbar_init(&acc_ready[h], 1);
+        }
         abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 0) tmem_alloc(&tmem_base, 256);
+    if (warp == 0) tmem_alloc(&tmem_base, 512);
     grid_wait();
     grid_trigger();
     for (int i = threadIdx.x; i < 4 * WIDTH; i += CH_THREADS) bias[i / WIDTH][i % WIDTH] = g.params[bias_at(i / WIDTH) + i % WIDTH];
@@ -207,77 +218,114 @@ __global__ void __launch_bounds__(CH_THREADS, 1) chain_kernel(ChainArgs g) {
                 if (!mbar_wait(&full[i % CH_STAGES], (i / CH_STAGES) & 1, WAIT_CYCLES)) flag_error(g.error, 102, &abort_flag);
         }
     } else if (warp == 17) {
-        constexpr uint32_t idesc = idesc_bf16(128, 256);
+        constexpr uint32_t idesc = idesc_bf16(128, 128);
         const bool leader = elect_one();
         const uint32_t act_addr = smem_u32(act), ring_addr = smem_u32(ring);
-        uint32_t chunk = 0;
+        uint32_t chunk = 0, seconds = 0;  // seconds: products so far that wait for the operand's second half
         bool ok = true;
-        for (uint32_t n = 0; n < 7 * turns && ok; n++) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&act_ready, n & 1, WAIT_CYCLES));
-            if (!ok) {
-                flag_error(g.error, 103, &abort_flag);
-                break;
+        auto wait = [&](uint64_t *bar, uint32_t parity, int code) {
+            if (ok && !__all_sync(0xffffffffu, mbar_wait(bar, parity, WAIT_CYCLES))) {
+                flag_error(g.error, code, &abort_flag);
+                ok = false;
             }
-            const int kts = n % 7 == 0 ? 1 : 4;
-            for (int kt = 0; kt < kts; kt++, chunk++) {
-                const int s = chunk % CH_STAGES;
-                ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (chunk / CH_STAGES) & 1, WAIT_CYCLES));
-                if (!ok) {
-                    flag_error(g.error, 104, &abort_flag);
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t a_addr = act_addr + kt * TILE_A, b_addr = ring_addr + s * CH_CHUNK;
-                if (leader) {
+        };
+        // one k tile of one column half of product n
+        auto issue = [&](uint32_t n, int kt, int h) {
+            const uint32_t a_addr = act_addr + kt * TILE_A, b_addr = ring_addr + (chunk + kt) % CH_STAGES * CH_CHUNK + h * TILE_A;
+            if (leader)
 #pragma unroll
-                    for (uint32_t k = 0; k < 4; k++)
-                        mma_bf16(tmem, sw128_desc(a_addr + 32 * k), sw128_desc(b_addr + 32 * k), idesc, (kt | k) != 0);
-                    mma_commit(&empty[s]);
-                    if (kt == kts - 1) mma_commit(&acc_ready);
+                for (uint32_t k = 0; k < 4; k++)
+                    mma_bf16(tmem + (n & 1) * 256 + h * 128, sw128_desc(a_addr + 32 * k), sw128_desc(b_addr + 32 * k), idesc,
+                             (kt | k) != 0);
+        };
+        auto commit = [&](uint64_t *bar) {
+            if (leader) mma_commit(bar);
+        };
+        for (uint32_t n = 0; n < 7 * turns && ok; n++) {
+            const int kts = n % 7 == 0 ? 1 : 4;
+            auto arrived = [&](int kt) {
+                wait(&full[(chunk + kt) % CH_STAGES], ((chunk + kt) / CH_STAGES) & 1, 104);
+                tc_fence_after();
+            };
+            wait(&act_ready[0], n & 1, 103);
+            if (kts == 4) {
+                for (int kt = 0; kt < 2 && ok; kt++) {
+                    arrived(kt);
+                    if (!ok) break;
+                    issue(n, kt, 0);
+                    issue(n, kt, 1);
+                    commit(&empty[(chunk + kt) % CH_STAGES]);
                 }
-                __syncwarp();
+                wait(&act_ready[1], seconds++ & 1, 103);
             }
+            for (int kt = kts == 4 ? 2 : 0; kt < kts && ok; kt++) {
+                arrived(kt);
+                if (ok) issue(n, kt, 0);
+            }
+            if (!ok) break;
+            if (kts == 1) issue(n, 0, 1);  // (it reads the half that the first epilogue replaces)
+            commit(&acc_ready[0]);
+            for (int kt = kts == 4 ? 2 : 0; kt < kts; kt++) {
+                if (kts == 4) issue(n, kt, 1);
+                commit(&empty[(chunk + kt) % CH_STAGES]);
+            }
+            commit(&acc_ready[1]);
+            __syncwarp();
+            chunk += kts;
         }
     } else {
-        const uint32_t c = warp >> 2, quarter = warp & 3, r = 32 * quarter + lane, col = 64 * c;
-        const uint32_t acc = tmem + ((uint32_t)(32 * quarter) << 16) + col;
+        const uint32_t c = warp >> 2, quarter = warp & 3, r = 32 * quarter + lane, col = 32 * c;
+        const uint32_t acc0 = tmem + ((uint32_t)(32 * quarter) << 16) + col;
         const bool first = threadIdx.x == 0;
-        uint8_t *mine = act + c * TILE_A;  // this thread's columns are one A tile's
-        uint32_t accs = 0;
+        uint32_t n = 0, acc = acc0;  // the product, and this thread's columns of its accumulator's first half
         // After a given-up wait the threads go on without waiting (every barrier is met; the outputs
         // are not used: the error is flagged).
-        auto wait_acc = [&]() {
-            if (!abort_flag && !mbar_wait(&acc_ready, accs & 1, WAIT_CYCLES)) flag_error(g.error, 105, &abort_flag);
-            accs++;
+        auto wait_acc = [&](int h) {
+            if (!abort_flag && !mbar_wait(&acc_ready[h], n & 1, WAIT_CYCLES)) flag_error(g.error, 105, &abort_flag);
+            acc = acc0 + (n & 1) * 256;
             __syncwarp();
             tc_fence_after();
-            // the activations' stores have read them: the epilogue may replace them
-            if (first) bulk_store_read();
-            epilogue_barrier();
         };
-        // the written operand is stored to `image` and, with `next`, handed to the next product
-        auto hand_over = [&](uint8_t *image, uint32_t bytes, bool next) {
+        // Half h of the written operand is stored to `image` and, with `next`, handed to the next
+        // product. The store before it, of the other half, has read its shared memory when the barrier
+        // is passed: that half may be replaced.
+        auto hand_over = [&](uint8_t *image, uint32_t bytes, int h, bool next) {
             fence_async_shared();
             tc_fence_before();
+            if (first) bulk_store_read();
             epilogue_barrier();
             if (first) {
-                if (next) mbar_arrive(&act_ready);
-                bulk_store(image, act, bytes);
+                if (next) mbar_arrive(&act_ready[h]);
+                bulk_store(image + h * 2 * TILE_A, act + h * 2 * TILE_A, bytes);
             }
         };
-        // the rows' sums of the 128 points, from the quarters' sums, into `out` [tile][256]
-        auto column_sums = [&](float (*part)[WIDTH], float *out, uint32_t tile) {
-            if (threadIdx.x < WIDTH)
-                out[(size_t)tile * WIDTH + threadIdx.x] =
-                    part[0][threadIdx.x] + part[1][threadIdx.x] + part[2][threadIdx.x] + part[3][threadIdx.x];
+        // 32 columns of half h of row r
+        auto store_columns = [&](int h, const uint32_t (&ph)[16]) {
+            uint8_t *tile = act + (2 * h + (c >> 1)) * TILE_A;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++)
+                *reinterpret_cast<uint4 *>(tile + sw128_offset(r, 32 * (c & 1) + 8 * q)) =
+                    make_uint4(ph[4 * q], ph[4 * q + 1], ph[4 * q + 2], ph[4 * q + 3]);
+        };
+        // The sums over the 128 points of half h's columns, from the quarters' sums, into `out`
+        // [tile][256]. The quarters' sums are taken behind the operand's hand-over, under the next
+        // product, and added up behind the hand-over after that.
+        auto column_sums = [&](float (*part)[WIDTH], float *out, uint32_t tile, int h) {
+            const uint32_t k = (threadIdx.x & 127) + 128 * h;
+            if (c == 3) out[(size_t)tile * WIDTH + k] = part[0][k] + part[1][k] + part[2][k] + part[3][k];
+        };
+        // this thread's Z of a layer's half h, asked for one half's epilogue ahead of its use
+        uint4 zs[4];
+        auto load_z = [&](int layer, uint32_t tile, int h) {
+            const uint4 *zt = g.z[layer] + ((size_t)tile * 8 + 4 * h) * CH_EPI + threadIdx.x;
+#pragma unroll
+            for (int q = 0; q < 4; q++) zs[q] = zt[q * CH_EPI];
         };
         for (uint32_t i = 0; i < turns; i++) {
             const uint32_t tile = blockIdx.x + i * gridDim.x, m = tile * 128 + r;
-            uint32_t ph[32];
+            uint32_t ph[16];
             // the inputs: features [16 c, 16 c + 16) of row r (K = 64)
             {
-                if (first) bulk_store_read();  // (the last tile's dZ1)
-                epilogue_barrier();
                 uint32_t p[8];
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
@@ -290,71 +338,55 @@ __global__ void __launch_bounds__(CH_THREADS, 1) chain_kernel(ChainArgs g) {
                 for (int q = 0; q < 2; q++)
                     *reinterpret_cast<uint4 *>(act + sw128_offset(r, 16 * c + 8 * q)) =
                         make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
-                hand_over(g.x_img + (size_t)tile * TILE_A, TILE_A, true);
+                hand_over(g.x_img + (size_t)tile * TILE_A, TILE_A, 0, true);
             }
             // layers 1-3 forward
-            for (int layer = 0; layer < 3; layer++) {
-                wait_acc();
+            for (int layer = 0; layer < 3; layer++, n++) {
                 uint4 *zt = g.z[layer] + (size_t)tile * 8 * CH_EPI + threadIdx.x;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     float v[32];
                     uint32_t pz[16];
-                    tmem_load32(acc + 32 * h, v);
+                    wait_acc(h);
+                    tmem_load32(acc + 128 * h, v);
 #pragma unroll
                     for (int j = 0; j < 32; j += 2) {
-                        const float z0 = v[j] + bias[layer][col + 32 * h + j], z1 = v[j + 1] + bias[layer][col + 32 * h + j + 1];
+                        const int k = 128 * h + col + j;
+                        const float z0 = v[j] + bias[layer][k], z1 = v[j + 1] + bias[layer][k + 1];
                         pz[j / 2] = pack_bf16(z0, z1);
-                        ph[16 * h + j / 2] = pack_bf16(silu(z0), silu(z1));
+                        ph[j / 2] = pack_bf16(silu(z0), silu(z1));
                     }
 #pragma unroll
                     for (int q = 0; q < 4; q++)
                         zt[(4 * h + q) * CH_EPI] = make_uint4(pz[4 * q], pz[4 * q + 1], pz[4 * q + 2], pz[4 * q + 3]);
+                    if (layer == 0 && h == 0) {  // X's store was the last one, and of the same half
+                        if (first) bulk_store_read();
+                        epilogue_barrier();
+                    }
+                    store_columns(h, ph);
+                    hand_over(g.h_img[layer] + (size_t)tile * 4 * TILE_A, 2 * TILE_A, h, true);
                 }
-                store_row(mine, r, ph);
-                hand_over(g.h_img[layer] + (size_t)tile * 4 * TILE_A, 4 * TILE_A, true);
             }
             // layer 4 and the output layer: out, dout, dZ4 = dout w5 silu'(z4)
-            wait_acc();
             {
                 float out = 0.0f;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     float v[32];
-                    tmem_load32(acc + 32 * h, v);
+                    wait_acc(h);
+                    tmem_load32(acc + 128 * h, v);
 #pragma unroll
                     for (int j = 0; j < 32; j += 2) {
-                        const int n = col + 32 * h + j;
-                        const uint32_t w = pack_bf16(silu(v[j] + bias[3][n]), silu(v[j + 1] + bias[3][n + 1]));
-                        out += __uint_as_float(w << 16) * w5[n];
-                        out += __uint_as_float(w & 0xffff0000u) * w5[n + 1];
+                        const int k = 128 * h + col + j;
+                        const uint32_t w = pack_bf16(silu(v[j] + bias[3][k]), silu(v[j + 1] + bias[3][k + 1]));
+                        out += __uint_as_float(w << 16) * w5[k];
+                        out += __uint_as_float(w & 0xffff0000u) * w5[k + 1];
                     }
                 }
                 dot[c][r] = out;
                 epilogue_barrier();
                 out = dot[0][r] + dot[1][r] + dot[2][r] + dot[3][r] + w5[WIDTH];
                 const float err = out - g.y[m], dout = 2.0f * err * g.inv_batch;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    float v[32], hw[32];
-                    tmem_load32(acc + 32 * h, v);
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const int n = col + 32 * h + j;
-                        const float z = v[j] + bias[3][n], t = tanh_fast(0.5f * z), s = 0.5f + 0.5f * t;
-                        hw[j] = fmaf(0.5f * z, t, 0.5f * z);
-                        v[j] = dout * w5[n] * (s * (1.0f + z * (1.0f - s)));
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; j += 2) {
-                        ph[16 * h + j / 2] = pack_bf16(v[j], v[j + 1]);
-                        const uint32_t w = pack_bf16(hw[j], hw[j + 1]);
-                        hw[j] = dout * __uint_as_float(w << 16);
-                        hw[j + 1] = dout * __uint_as_float(w & 0xffff0000u);
-                    }
-                    part_a[quarter][col + 32 * h + lane] = warp_column_sum(v);
-                    part_b[quarter][col + 32 * h + lane] = warp_column_sum(hw);
-                }
                 if (c == 0) {
                     float a = dout, b = err * err;
 #pragma unroll
@@ -367,48 +399,77 @@ __global__ void __launch_bounds__(CH_THREADS, 1) chain_kernel(ChainArgs g) {
                         scal[quarter][1] = b;
                     }
                 }
-                store_row(mine, r, ph);
-                hand_over(g.dz_img[3] + (size_t)tile * 4 * TILE_A, 4 * TILE_A, true);
-                column_sums(part_a, g.db[3], tile);
-                column_sums(part_b, g.dw5, tile);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    float v[32], hw[32];
+                    tmem_load32(acc + 128 * h, v);
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {
+                        const int k = 128 * h + col + j;
+                        const float z = v[j] + bias[3][k], t = tanh_fast(0.5f * z), s = 0.5f + 0.5f * t;
+                        hw[j] = fmaf(0.5f * z, t, 0.5f * z);
+                        v[j] = dout * w5[k] * (s * (1.0f + z * (1.0f - s)));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        ph[j / 2] = pack_bf16(v[j], v[j + 1]);
+                        const uint32_t w = pack_bf16(hw[j], hw[j + 1]);
+                        hw[j] = dout * __uint_as_float(w << 16);
+                        hw[j + 1] = dout * __uint_as_float(w & 0xffff0000u);
+                    }
+                    store_columns(h, ph);
+                    hand_over(g.dz_img[3] + (size_t)tile * 4 * TILE_A, 2 * TILE_A, h, true);
+                    if (h == 1) {
+                        load_z(2, tile, 0);
+                        column_sums(part_a, g.db[3], tile, 0);
+                        column_sums(part_b, g.dw5, tile, 0);
+                    }
+                    part_a[quarter][128 * h + col + lane] = warp_column_sum(v);
+                    part_b[quarter][128 * h + col + lane] = warp_column_sum(hw);
+                }
                 if (threadIdx.x < 2)
                     g.scalars[2 * tile + threadIdx.x] =
                         scal[0][threadIdx.x] + scal[1][threadIdx.x] + scal[2][threadIdx.x] + scal[3][threadIdx.x];
+                n++;
             }
             // back: dZ3, dZ2, dZ1
-            for (int layer = 2; layer >= 0; layer--) {
-                uint4 zs[8];
-                const uint4 *zt = g.z[layer] + (size_t)tile * 8 * CH_EPI + threadIdx.x;
-#pragma unroll
-                for (int q = 0; q < 8; q++) zs[q] = zt[q * CH_EPI];
-                wait_acc();
+            for (int layer = 2; layer >= 0; layer--, n++) {
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     float v[32];
-                    tmem_load32(acc + 32 * h, v);
+                    uint4 z[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) z[q] = zs[q];
+                    if (h == 0) load_z(layer, tile, 1);
+                    else if (layer > 0) load_z(layer - 1, tile, 0);
+                    wait_acc(h);
+                    tmem_load32(acc + 128 * h, v);
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        const uint32_t ws[4] = {zs[4 * h + q].x, zs[4 * h + q].y, zs[4 * h + q].z, zs[4 * h + q].w};
+                        const uint32_t ws[4] = {z[q].x, z[q].y, z[q].z, z[q].w};
 #pragma unroll
                         for (int e = 0; e < 4; e++) {
                             v[8 * q + 2 * e] *= silu_grad(__uint_as_float(ws[e] << 16));
                             v[8 * q + 2 * e + 1] *= silu_grad(__uint_as_float(ws[e] & 0xffff0000u));
-                            ph[16 * h + 4 * q + e] = pack_bf16(v[8 * q + 2 * e], v[8 * q + 2 * e + 1]);
+                            ph[4 * q + e] = pack_bf16(v[8 * q + 2 * e], v[8 * q + 2 * e + 1]);
                         }
                     }
-                    part_a[quarter][col + 32 * h + lane] = warp_column_sum(v);
+                    store_columns(h, ph);
+                    hand_over(g.dz_img[layer] + (size_t)tile * 4 * TILE_A, 2 * TILE_A, h, layer > 0);
+                    column_sums(part_a, g.db[h ? layer : layer + 1], tile, 1 - h);
+                    if (layer == 2 && h == 0) column_sums(part_b, g.dw5, tile, 1);
+                    part_a[quarter][128 * h + col + lane] = warp_column_sum(v);
                 }
-                store_row(mine, r, ph);
-                hand_over(g.dz_img[layer] + (size_t)tile * 4 * TILE_A, 4 * TILE_A, layer > 0);
-                column_sums(part_a, g.db[layer], tile);
             }
+            epilogue_barrier();
+            column_sums(part_a, g.db[0], tile, 1);
         }
         if (first) bulk_store_done();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) tmem_dealloc(tmem, 256);
+    if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 // ---- the weight gradients -------------------------------------------------------------------------
