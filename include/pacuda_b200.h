@@ -82,7 +82,8 @@ int pacuda_b200_batch_capture(pacuda_b200_batch *batch, void *stream);
  * shared memory (while one waits at a level's barrier the others run); 0: chosen per plan without
  * timing (four for a plan of at most four points per 16-warp block, else two). Replaces the tuner's
  * per-plan choices. INVALID for another count or when the plans' points do not fit. A new batch
- * has 1. */
+ * has 1. With 0 or 1, and no choice given per plan, a batch of at most one point per SM in all may
+ * run one point per block and one block per SM in one launch (the same values). */
 int pacuda_b200_batch_set_blocks_per_sm(pacuda_b200_batch *batch, uint32_t blocks);
 uint32_t pacuda_b200_batch_blocks_per_sm(const pacuda_b200_batch *batch);
 /* the blocks per SM plan k runs with (its own choice, else the batch's); setting 0 returns it to

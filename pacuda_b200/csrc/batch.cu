@@ -51,6 +51,7 @@ struct pacuda_b200_plan {
     uint32_t points = 1;      // points per block (a point has the block's threads / points lanes)
     size_t point_bytes = 0;
     bool fixed = false;
+    bool wide = false;  // a level has more tasks than a point's default lanes
 };
 
 // The plans of one launch: those that run with the same blocks per SM.
@@ -68,12 +69,15 @@ struct pacuda_b200_batch {
     std::vector<double *> output;
     std::vector<uint32_t> points;      // per plan: its points per block in this batch's launch
     std::vector<int> plan_blocks;      // per plan: its blocks per SM (0: the batch's)
+    std::vector<uint8_t> given;        // per plan: whether the caller gave its blocks per SM
     int blocks = 1;                    // the batch's blocks per SM (tiled_host.h kBlockChoices); 0: automatic
+    bool spread = true;                // a few points are spread over the SMs (few_points; not in timings)
+    int tuned_few = 0;                 // a tuned plan by itself: whether that was faster (1) or not (-1)
     // one launch per group; the descriptor block holds a section per group:
     // TiledPlan[n] | item_first[n + 1] | external[n] | output[n] | count[n] | counter
     std::vector<LaunchGroup> groups;
     unsigned char *host = nullptr, *device = nullptr;
-    size_t bytes = 0;
+    size_t bytes = 0;                  // in use, of a size for a group per plan
     int sms = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -130,15 +134,38 @@ size_t group_const_bytes(pacuda_b200_plan *const *plans, const uint32_t *which, 
     return table + point <= tiled_max_smem(kernel, blocks) ? table : 0;
 }
 
+// Few points: a batch that has no more points, in all its plans, than the GPU has SMs can run one
+// point per block and one block per SM, in one launch: each point has an SM and all its warps to
+// itself, where the other choices share an SM's warps and leave SMs idle. It does where a level of a
+// plan has more tasks than a point's default lanes, and the launch is not given by the caller; a
+// tuned plan by itself, where that was faster than its best pair. (64 points, B200: gg>ggg f64 30.6
+// -> 18.8 us (its best pair 20.4), mixed 34.9 -> 18.6 (24.8), df64 106 -> 54 (78); qg>qgg f64 26.9
+// -> 18.5 (22.6); qq~>gg, whose levels are narrow, 14.0 -> 15.7 (12.5). At 250 points, above the
+// line: gg>ggg 30.6 against 20.6 for its best pair.)
+bool few_points(const pacuda_b200_batch *b) {
+    if (!b->spread || b->blocks > 1) return false;
+    uint64_t total = 0;
+    bool wide = false;
+    for (size_t k = 0; k < b->plans.size(); k++) {
+        if (b->plans[k]->fixed || b->given[k]) return false;
+        total += b->count[k];
+        wide = wide || b->plans[k]->wide;
+    }
+    if (total > (uint64_t)b->sms) return false;
+    return b->plans.size() == 1 && b->tuned_few ? b->tuned_few > 0 : wide;
+}
+
 // The groups and the host block from the batch's current choices: each group's shared memory and
-// warps, each plan's points per block. The block is allocated again only when its size changes.
+// warps, each plan's points per block.
 bool prepare(pacuda_b200_batch *b) {
     const size_t n = b->plans.size();
     const int kernel = b->plans[0]->kernel;
     b->plan_blocks.resize(n, 0);
+    b->given.resize(n, 0);
     b->groups.clear();
+    const bool few = few_points(b);
     for (size_t k = 0; k < n; k++) {
-        int blocks = b->plan_blocks[k] ? b->plan_blocks[k] : b->blocks ? b->blocks : auto_blocks(b->plans[k]);
+        int blocks = few ? 1 : b->plan_blocks[k] ? b->plan_blocks[k] : b->blocks ? b->blocks : auto_blocks(b->plans[k]);
         size_t g = 0;
         while (g < b->groups.size() && b->groups[g].blocks != blocks) g++;
         if (g == b->groups.size()) {
@@ -152,14 +179,11 @@ bool prepare(pacuda_b200_batch *b) {
         g.at = bytes;
         bytes += layout(g.plans.size()).total;
     }
-    if (!b->host || bytes != b->bytes) {
-        cudaFreeHost(b->host);
-        cudaFree(b->device);
-        b->host = nullptr;
-        b->device = nullptr;
-        b->bytes = bytes;
-        if (failed(cudaMallocHost((void **)&b->host, b->bytes), "pinned descriptors") ||
-            failed(cudaMalloc((void **)&b->device, b->bytes), "descriptors"))
+    b->bytes = bytes;
+    if (!b->host) {  // (once: an update that changes the groups allocates nothing)
+        const size_t most = n * layout(1).total;
+        if (failed(cudaMallocHost((void **)&b->host, most), "pinned descriptors") ||
+            failed(cudaMalloc((void **)&b->device, most), "descriptors"))
             return false;
     }
     memset(b->host, 0, b->bytes);
@@ -184,7 +208,7 @@ bool prepare(pacuda_b200_batch *b) {
                 return false;
             }
             // the plan's choice where it fits this launch, else the default for it
-            uint32_t per = tiled_points_fit(p->points, p->point_bytes, g.threads, max_smem)
+            uint32_t per = few ? 1 : tiled_points_fit(p->points, p->point_bytes, g.threads, max_smem)
                                ? p->points
                                : tiled_default_points(p->point_bytes, g.threads, max_smem);
             b->points[k] = per;
@@ -334,6 +358,9 @@ extern "C" pacuda_b200_plan *pacuda_b200_plan_create(const pacman_recurrence_cal
     }
     p->point_bytes = tiled_point_bytes(p->tiled, forms, p->kernel);
     p->points = default_points(p);
+    const std::vector<uint32_t> &first = p->tiled.host.level_first;
+    for (size_t l = 0; l + 1 < first.size(); l++)
+        p->wide = p->wide || first[l + 1] - first[l] > tiled_lanes(p->points, tiled_threads(p->kernel));
     return p;
 }
 
@@ -474,6 +501,7 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
         float ms = -1.0f;
         if (tb) {
             tb->blocks = blocks;
+            tb->spread = false;
             bool ok = prepare(tb) && tb->points[0] == points && launch(tb, s) == PACMAN_RECURRENCE_OK;
             for (int rep = 0; ok && rep < 3; rep++) {
                 cudaEventRecord(t0, s);
@@ -514,6 +542,10 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
                 }
             }
         }
+        if (best >= 0.0f && b->plans.size() == 1 && b->count[0] <= (uint32_t)b->sms) {
+            const float few = time_plan(0, 1, 1);
+            b->tuned_few = few >= 0.0f && few < best ? 1 : -1;
+        }
         if (best >= 0.0f) {
             p->points = best_points;
             b->plan_blocks[k] = best_blocks;
@@ -543,11 +575,14 @@ extern "C" int pacuda_b200_batch_set_blocks_per_sm(pacuda_b200_batch *b, uint32_
     }
     int before = b->blocks;
     std::vector<int> before_plans = b->plan_blocks;
+    std::vector<uint8_t> before_given = b->given;
     b->blocks = (int)blocks;
     std::fill(b->plan_blocks.begin(), b->plan_blocks.end(), 0);  // every plan the same
+    std::fill(b->given.begin(), b->given.end(), 0);
     if (!prepare(b)) {
         b->blocks = before;
         b->plan_blocks = before_plans;
+        b->given = before_given;
         prepare(b);
         return PACMAN_RECURRENCE_INVALID;
     }
@@ -566,9 +601,12 @@ extern "C" int pacuda_b200_batch_set_plan_blocks_per_sm(pacuda_b200_batch *b, ui
         b->graph = nullptr;
     }
     int before = b->plan_blocks[plan];
+    uint8_t before_given = b->given[plan];
     b->plan_blocks[plan] = (int)blocks;
+    b->given[plan] = blocks != 0;
     if (!prepare(b)) {
         b->plan_blocks[plan] = before;
+        b->given[plan] = before_given;
         prepare(b);
         return PACMAN_RECURRENCE_INVALID;
     }
