@@ -65,7 +65,8 @@ pacuda_b200_batch *pacuda_b200_batch_create(pacuda_b200_plan *const *plans, uint
                                             double *const *output);
 /* Points the batch's plans at other arrays and point counts (as batch_create takes them), without
  * allocating; a captured graph is dropped (capture again to replay). Waits for the previous run's
- * copy of the launch descriptors, not for its kernel: the caller orders its use of the old arrays. */
+ * copy of the launch descriptors, not for its kernel (of a captured batch: for its last replay): the
+ * caller orders its use of the old arrays. */
 int pacuda_b200_batch_update(pacuda_b200_batch *batch, const double *const *external, const uint32_t *count,
                              double *const *output);
 /* Times each plan's lanes-per-point choices on its own points, with 1, 2, 3, 4, 5, 8 and 16 blocks

@@ -81,7 +81,9 @@ struct pacuda_b200_batch {
     int sms = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    cudaEvent_t copied = nullptr;  // recorded after each run's descriptor copy
+    // the host block's last reader on the device: recorded after each run's descriptor copy, and after
+    // each replay of the captured graph, whose copy node reads the block when the replay's turn comes
+    cudaEvent_t copied = nullptr;
 };
 
 namespace {
@@ -242,13 +244,20 @@ TiledLaunch launch_args(const pacuda_b200_batch *b, const LaunchGroup &g) {
     return L;
 }
 
-int launch(pacuda_b200_batch *b, cudaStream_t s) {
-    if (failed(cudaMemcpyAsync(b->device, b->host, b->bytes, cudaMemcpyHostToDevice, s), "descriptors"))
-        return PACMAN_RECURRENCE_DEVICE_ERROR;
-    // (not while capturing: the graph's copy reads the block when it is replayed)
+// the work of `s` so far reads the host block (nothing is read while `s` is captured: a graph's copy
+// reads the block when it is replayed)
+bool record_copied(pacuda_b200_batch *b, cudaStream_t s) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(s, &capturing);
-    if (capturing == cudaStreamCaptureStatusNone && b->copied && failed(cudaEventRecord(b->copied, s), "event"))
+    return capturing != cudaStreamCaptureStatusNone || !failed(cudaEventRecord(b->copied, s), "event");
+}
+
+// before the host block is written again
+bool wait_copied(pacuda_b200_batch *b) { return !failed(cudaEventSynchronize(b->copied), "descriptors"); }
+
+int launch(pacuda_b200_batch *b, cudaStream_t s) {
+    if (failed(cudaMemcpyAsync(b->device, b->host, b->bytes, cudaMemcpyHostToDevice, s), "descriptors") ||
+        !record_copied(b, s))
         return PACMAN_RECURRENCE_DEVICE_ERROR;
     for (const LaunchGroup &g : b->groups)
         if (!launch_tiled(b->plans[0]->kernel, launch_args(b, g), g.threads, g.smem, b->sms * g.blocks, s) ||
@@ -431,8 +440,7 @@ extern "C" int pacuda_b200_batch_update(pacuda_b200_batch *b, const double *cons
             fprintf(stderr, "%s: batch_update: plan %zu: a missing array or point count\n", kTag, k);
             return PACMAN_RECURRENCE_INVALID;
         }
-    // the previous launch's copy of the descriptors must have left the pinned block
-    if (failed(cudaEventSynchronize(b->copied), "batch_update")) return PACMAN_RECURRENCE_DEVICE_ERROR;
+    if (!wait_copied(b)) return PACMAN_RECURRENCE_DEVICE_ERROR;
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
         cudaGraphDestroy(b->graph);
@@ -449,8 +457,9 @@ extern "C" int pacuda_b200_batch_update(pacuda_b200_batch *b, const double *cons
 extern "C" int pacuda_b200_batch_run(pacuda_b200_batch *b, void *stream) {
     if (!b) return PACMAN_RECURRENCE_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
-    if (b->exec) return failed(cudaGraphLaunch(b->exec, s), "graph") ? PACMAN_RECURRENCE_DEVICE_ERROR : PACMAN_RECURRENCE_OK;
-    return launch(b, s);
+    if (!b->exec) return launch(b, s);
+    return failed(cudaGraphLaunch(b->exec, s), "graph") || !record_copied(b, s) ? PACMAN_RECURRENCE_DEVICE_ERROR
+                                                                                 : PACMAN_RECURRENCE_OK;
 }
 
 extern "C" int pacuda_b200_batch_capture(pacuda_b200_batch *b, void *stream) {
@@ -553,6 +562,7 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
     }
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
+    if (!wait_copied(b)) return PACMAN_RECURRENCE_DEVICE_ERROR;
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
         cudaGraphDestroy(b->graph);
@@ -566,7 +576,7 @@ extern "C" uint32_t pacuda_b200_batch_launches(const pacuda_b200_batch *b) { ret
 
 extern "C" int pacuda_b200_batch_set_blocks_per_sm(pacuda_b200_batch *b, uint32_t blocks) {
     if (!b || (blocks && !tiled_blocks_valid((int)blocks))) return PACMAN_RECURRENCE_INVALID;
-    if (failed(cudaEventSynchronize(b->copied), "batch")) return PACMAN_RECURRENCE_DEVICE_ERROR;
+    if (!wait_copied(b)) return PACMAN_RECURRENCE_DEVICE_ERROR;
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
         cudaGraphDestroy(b->graph);
@@ -593,7 +603,7 @@ extern "C" uint32_t pacuda_b200_batch_blocks_per_sm(const pacuda_b200_batch *b) 
 
 extern "C" int pacuda_b200_batch_set_plan_blocks_per_sm(pacuda_b200_batch *b, uint32_t plan, uint32_t blocks) {
     if (!b || plan >= b->plans.size() || (blocks && !tiled_blocks_valid((int)blocks))) return PACMAN_RECURRENCE_INVALID;
-    if (failed(cudaEventSynchronize(b->copied), "batch")) return PACMAN_RECURRENCE_DEVICE_ERROR;
+    if (!wait_copied(b)) return PACMAN_RECURRENCE_DEVICE_ERROR;
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
         cudaGraphDestroy(b->graph);
