@@ -142,12 +142,12 @@ struct ChainArgs {
 };
 
 // A training step's three kernels are launched ahead of their turn (launch_early): a block sets up
-// its barriers and tensor memory, and the update its parameters, while the kernel before runs out.
-// grid_wait: until that kernel is complete and its writes are seen; everything that an earlier kernel
-// wrote, or still reads, is touched behind it. grid_trigger: the next kernel's blocks may be placed. Every
-// block triggers behind its own wait, so a placed kernel knows that the one before the one it waits
-// for is complete (what the update loads ahead was written by the step before).
-// 16 steps of 16 384 points: 1264 -> 1135 us (8 us of a step's 79 were the three kernels' ends and starts).
+// its barriers and tensor memory while the kernel before runs out. grid_wait: until that kernel is
+// complete and its writes, and those of every kernel before it, are seen; all that another kernel
+// writes or reads is touched behind it. grid_trigger, behind the block's own wait: the next kernel's
+// blocks may be placed, so a placed kernel has at most one unfinished kernel before it.
+// 16 steps of 16 384 points: 1264 -> 1135 us (8 us of a step's 79 were the three kernels' ends and starts); the
+// update's own loads of the parameters ahead of the wait gave none of it (1043 us with and without).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -671,13 +671,13 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs u) {
         const uint32_t o = row0 + y, c4 = first4 + x;
         const size_t t = (layer == 0 ? P_W1 : layer == 1 ? P_W2 : layer == 2 ? P_W3 : P_W4) + (size_t)o * fan + 4 * c4;
         float4 w, a, b;
-        if (MODE != UP_GRADIENT) {  // (the network's own arrays: aligned)
+        grid_wait();
+        grid_trigger();
+        if (MODE != UP_GRADIENT) {  // (the network's own arrays: aligned; they come while the partials are summed)
             w = *reinterpret_cast<const float4 *>(u.params + t);
             a = *reinterpret_cast<const float4 *>(u.m1 + t);
             b = *reinterpret_cast<const float4 *>(u.m2 + t);
         }
-        grid_wait();
-        grid_trigger();
         float4 g;
         if (MODE != UP_APPLY) {
             const float4 *p = reinterpret_cast<const float4 *>(u.dw[layer]) + (size_t)(first4 + y) * WIDTH + row0 + x;
@@ -1406,7 +1406,7 @@ template <int MODE> int update(pacuda_sg_net *n, UpdateArgs &u, float lr, cudaSt
         u.c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)n->step)));
     }
     if (MODE != UP_APPLY) return launch_early(update_kernel<MODE>, UP_BLOCKS, 256, 0, s, u, "update") ? ST_OK : ST_DEVICE;
-    // (after another kernel than this step's the parameters that it loads before it waits may not be in)
+    // (a call of its own, after whatever the caller queued)
     update_kernel<MODE><<<UP_BLOCKS, 256, 0, s>>>(u);
     g_last_launches++;
     return failed(cudaGetLastError(), "update") ? ST_DEVICE : ST_OK;
