@@ -72,7 +72,9 @@ int pacuda_b200_batch_update(pacuda_b200_batch *batch, const double *const *exte
 /* Times each plan's lanes-per-point choices on its own points, with 1, 2, 3, 4, 5, 8 and 16 blocks
  * per SM (those its points fit), and
  * keeps each plan's fastest pair; plans of the same blocks per SM share one launch (a run is then
- * one launch per blocks-per-SM choice in use, one after the other on the stream). */
+ * one launch per blocks-per-SM choice in use, one after the other on the stream). A batch of at most
+ * one point per SM in all is then timed at these pairs and, in one launch, at one point per block and
+ * one block per SM; where the latter is faster it runs so at these point counts. */
 int pacuda_b200_batch_tune(pacuda_b200_batch *batch, void *stream);
 /* One persistent launch over every plan's points, on `stream` (a cudaStream_t; NULL: default). */
 int pacuda_b200_batch_run(pacuda_b200_batch *batch, void *stream);
@@ -83,8 +85,9 @@ int pacuda_b200_batch_capture(pacuda_b200_batch *batch, void *stream);
  * shared memory (while one waits at a level's barrier the others run); 0: chosen per plan without
  * timing (four for a plan of at most four points per 16-warp block, else two). Replaces the tuner's
  * per-plan choices. INVALID for another count or when the plans' points do not fit. A new batch
- * has 1. With 0 or 1, and no choice given per plan, a batch of at most one point per SM in all may
- * run one point per block and one block per SM in one launch (the same values). */
+ * has 1. A batch of at most one point per SM in all that is not tuned, and whose choice is 0 or a new
+ * batch's own 1, none given per plan, may run one point per block and one block per SM in one launch
+ * (the same values). */
 int pacuda_b200_batch_set_blocks_per_sm(pacuda_b200_batch *batch, uint32_t blocks);
 uint32_t pacuda_b200_batch_blocks_per_sm(const pacuda_b200_batch *batch);
 /* the blocks per SM plan k runs with (its own choice, else the batch's); setting 0 returns it to

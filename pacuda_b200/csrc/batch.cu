@@ -71,8 +71,10 @@ struct pacuda_b200_batch {
     std::vector<int> plan_blocks;      // per plan: its blocks per SM (0: the batch's)
     std::vector<uint8_t> given;        // per plan: whether the caller gave its blocks per SM
     int blocks = 1;                    // the batch's blocks per SM (tiled_host.h kBlockChoices); 0: automatic
-    bool spread = true;                // a few points are spread over the SMs (few_points; not in timings)
-    int tuned_few = 0;                 // a tuned plan by itself: whether that was faster (1) or not (-1)
+    bool asked = false;                // whether the caller gave them (a new batch's 1 and the automatic 0 are not)
+    bool spread = true;                // a few points may be spread over the SMs (few_points; not in timings)
+    // the counts that the tuner timed spread over the SMs and found faster so than at its pairs
+    std::vector<uint32_t> spread_counts;
     // one launch per group; the descriptor block holds a section per group:
     // TiledPlan[n] | item_first[n + 1] | external[n] | output[n] | count[n] | counter
     std::vector<LaunchGroup> groups;
@@ -138,23 +140,25 @@ size_t group_const_bytes(pacuda_b200_plan *const *plans, const uint32_t *which, 
 
 // Few points: a batch that has no more points, in all its plans, than the GPU has SMs can run one
 // point per block and one block per SM, in one launch: each point has an SM and all its warps to
-// itself, where the other choices share an SM's warps and leave SMs idle. It does where a level of a
-// plan has more tasks than a point's default lanes, and the launch is not given by the caller; a
-// tuned plan by itself, where that was faster than its best pair. (64 points, B200: gg>ggg f64 30.6
-// -> 18.8 us (its best pair 20.4), mixed 34.9 -> 18.6 (24.8), df64 106 -> 54 (78); qg>qgg f64 26.9
-// -> 18.5 (22.6); qq~>gg, whose levels are narrow, 14.0 -> 15.7 (12.5). At 250 points, above the
-// line: gg>ggg 30.6 against 20.6 for its best pair.)
+// itself, where the other choices share an SM's warps and leave SMs idle. Never where the caller gave
+// the launch. A tuned batch does so for the counts at which the tuner measured it to be faster (at
+// others its pairs stand); one that is not tuned where a level of a plan has more tasks than a
+// point's default lanes. (64 points, B200: gg>ggg f64 30.6 -> 18.8 us (its best pair 20.4), mixed
+// 34.9 -> 18.6 (24.8), df64 106 -> 54 (78); qg>qgg f64 26.9 -> 18.5 (22.6); qq~>gg, whose levels are
+// narrow, 14.0 -> 15.7 (12.5). At 250 points, above the line: gg>ggg 30.6 against 20.6 for its best
+// pair.)
 bool few_points(const pacuda_b200_batch *b) {
-    if (!b->spread || b->blocks > 1) return false;
+    if (!b->spread || b->asked) return false;
     uint64_t total = 0;
-    bool wide = false;
+    bool wide = false, tuned = false;
     for (size_t k = 0; k < b->plans.size(); k++) {
         if (b->plans[k]->fixed || b->given[k]) return false;
         total += b->count[k];
         wide = wide || b->plans[k]->wide;
+        tuned = tuned || b->plan_blocks[k];
     }
     if (total > (uint64_t)b->sms) return false;
-    return b->plans.size() == 1 && b->tuned_few ? b->tuned_few > 0 : wide;
+    return tuned ? b->spread_counts == b->count : wide;
 }
 
 // The groups and the host block from the batch's current choices: each group's shared memory and
@@ -551,17 +555,12 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
                 }
             }
         }
-        if (best >= 0.0f && b->plans.size() == 1 && b->count[0] <= (uint32_t)b->sms) {
-            const float few = time_plan(0, 1, 1);
-            b->tuned_few = few >= 0.0f && few < best ? 1 : -1;
-        }
         if (best >= 0.0f) {
             p->points = best_points;
             b->plan_blocks[k] = best_blocks;
+            b->given[k] = 0;  // (the choice is the tuner's now)
         }
     }
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
     if (!wait_copied(b)) return PACMAN_RECURRENCE_DEVICE_ERROR;
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
@@ -569,7 +568,31 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
         b->exec = nullptr;
         b->graph = nullptr;
     }
-    return prepare(b) ? PACMAN_RECURRENCE_OK : PACMAN_RECURRENCE_DEVICE_ERROR;
+    // a batch of few points: all of it at its pairs and spread over the SMs, the best of three each
+    b->spread_counts = b->count;
+    if (few_points(b)) {
+        float ms[2] = {-1.0f, -1.0f};
+        for (int spread = 0; spread < 2; spread++) {
+            b->spread_counts = spread ? b->count : std::vector<uint32_t>();
+            bool ok = wait_copied(b) && prepare(b) && launch(b, s) == PACMAN_RECURRENCE_OK;
+            for (int rep = 0; ok && rep < 3; rep++) {
+                cudaEventRecord(t0, s);
+                ok = launch(b, s) == PACMAN_RECURRENCE_OK;
+                cudaEventRecord(t1, s);
+                cudaEventSynchronize(t1);
+                float m = 0;
+                cudaEventElapsedTime(&m, t0, t1);
+                ms[spread] = rep == 0 ? m : std::min(ms[spread], m);
+            }
+            if (!ok) ms[spread] = -1.0f;
+        }
+        if (ms[1] < 0.0f || (ms[0] >= 0.0f && ms[0] <= ms[1])) b->spread_counts.clear();
+    } else {
+        b->spread_counts.clear();
+    }
+    cudaEventDestroy(t0);
+    cudaEventDestroy(t1);
+    return wait_copied(b) && prepare(b) ? PACMAN_RECURRENCE_OK : PACMAN_RECURRENCE_DEVICE_ERROR;
 }
 
 extern "C" uint32_t pacuda_b200_batch_launches(const pacuda_b200_batch *b) { return b ? (uint32_t)b->groups.size() : 0; }
@@ -584,15 +607,21 @@ extern "C" int pacuda_b200_batch_set_blocks_per_sm(pacuda_b200_batch *b, uint32_
         b->graph = nullptr;
     }
     int before = b->blocks;
+    const bool before_asked = b->asked;
     std::vector<int> before_plans = b->plan_blocks;
     std::vector<uint8_t> before_given = b->given;
+    std::vector<uint32_t> before_spread = b->spread_counts;
     b->blocks = (int)blocks;
+    b->asked = blocks != 0;
+    b->spread_counts.clear();
     std::fill(b->plan_blocks.begin(), b->plan_blocks.end(), 0);  // every plan the same
     std::fill(b->given.begin(), b->given.end(), 0);
     if (!prepare(b)) {
         b->blocks = before;
+        b->asked = before_asked;
         b->plan_blocks = before_plans;
         b->given = before_given;
+        b->spread_counts = before_spread;
         prepare(b);
         return PACMAN_RECURRENCE_INVALID;
     }
@@ -612,11 +641,14 @@ extern "C" int pacuda_b200_batch_set_plan_blocks_per_sm(pacuda_b200_batch *b, ui
     }
     int before = b->plan_blocks[plan];
     uint8_t before_given = b->given[plan];
+    std::vector<uint32_t> before_spread = b->spread_counts;
     b->plan_blocks[plan] = (int)blocks;
     b->given[plan] = blocks != 0;
+    b->spread_counts.clear();  // (measured with another choice)
     if (!prepare(b)) {
         b->plan_blocks[plan] = before;
         b->given[plan] = before_given;
+        b->spread_counts = before_spread;
         prepare(b);
         return PACMAN_RECURRENCE_INVALID;
     }
@@ -775,7 +807,8 @@ extern "C" int pacuda_b200_run_static(pacuda_b200_plan *const *plans, uint32_t n
         }
     unsigned char *scratch = static_scratch();
     if (!scratch) return PACMAN_RECURRENCE_DEVICE_ERROR;
-    // the launch's shape as a batch of these plans has it; the plans' own choices are not changed
+    // the launch's shape as a batch of these plans at one block per SM has it (its rule for few points
+    // is not applied); the plans' own choices are not changed
     int kernel = plans[0]->kernel;
     int threads = tiled_threads(kernel);
     // the shared memory a block may have, less the plan constants every block holds (checked
