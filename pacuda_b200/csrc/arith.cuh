@@ -108,6 +108,7 @@ template <class R_, class Den_, class Amp_, class Const_> struct Kind {
     typedef Den_ Den;
     typedef Amp_ Amp;
     typedef Const_ Const;
+    static constexpr bool contracted = false;  // multiply-adds with one rounding (tiled_fma.cu)
 };
 typedef Kind<double, double, double, double> KindF64;
 typedef Kind<D, D, D, D> KindDF64;

@@ -622,6 +622,7 @@ __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
     typedef typename K::Amp Amp;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ unsigned long long next_item[2];  // by turns: this item and (AHEAD) the one after it
+    __shared__ uint32_t again;                   // (contracted) the item's points that are computed again, a bit each
     // The block's shared memory from its address in a register: taken from the array's symbol, every
     // row computes that address again (6 of 190 instructions; gg>ggg 4096 points 146 -> 143 us,
     // qg>qgg 125 -> 130 M points/s). The C ABI's kernel has no register left for it.
@@ -750,7 +751,8 @@ __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
                         ((Amp *)L.are)[plane * L.ld + at] = re;
                         ((Amp *)L.aim)[plane * L.ld + at] = im;
                     }
-            } else if (active && (size_t)(item - L.item_first[k]) * np + pw < L.count[k]) {
+            } else if (active && (size_t)(item - L.item_first[k]) * np + pw < L.count[k] &&
+                       (!K::contracted || !plain || again >> pw & 1)) {
                 // the resolved reduction from zero: out[point][o] = 0 + w fma(re, re, im im) + ...
                 const size_t point = (size_t)(item - L.item_first[k]) * np + pw;
                 double *out = L.output[k] + point * p.outputs;
@@ -784,6 +786,14 @@ __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
                 break;
             }
             if (!__syncthreads_or(bad) || plain) break;
+            // With contracted multiply-adds the plain formulas round otherwise: only those points' outputs are
+            // replaced, so that a point's bits do not depend on the points beside it. (In the other kinds a
+            // finite point gets the same bits again, and df64 has no registers to spare.)
+            if (K::contracted) {
+                if (threadIdx.x == 0) again = 0;
+                __syncthreads();
+                if (bad) atomicOr(&again, 1u << pw);
+            }
             plain = H_PLAIN;
         }
     }

@@ -8,7 +8,9 @@
 namespace pacuda {
 
 // a kind of its own (so that its kernels are not the -fmad=false f64 kind's instantiations)
-struct KindF64Fma : Kind<double, double, double, double> {};
+struct KindF64Fma : Kind<double, double, double, double> {
+    static constexpr bool contracted = true;
+};
 
 const void *tiled_fma_kernel(bool abi) {
     return abi ? (const void *)run_tiled<KindF64Fma, true> : (const void *)run_tiled<KindF64Fma, false>;
