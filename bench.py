@@ -39,6 +39,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -56,6 +57,19 @@ ECM = 13000.0
 SEED = 20261203
 TILE = 1 << 16
 OVERWEIGHT = 1e-3  # reduced unweighting maxima: at most this share of the total above them
+
+
+def json_line(value):
+    """`value` as one line of strict JSON: a number that is not finite (a ratio over an empty sample) is
+    null, which JSON has no other form for."""
+    def finite(v):
+        if isinstance(v, dict):
+            return {k: finite(x) for k, x in v.items()}
+        if isinstance(v, (list, tuple)):
+            return [finite(x) for x in v]
+        return None if isinstance(v, float) and not math.isfinite(v) else v
+
+    return json.dumps(finite(value), allow_nan=False)
 
 
 def split_points(total, seed):
@@ -805,7 +819,7 @@ def reference_gpu_worker(kind, steps, warmup, keep_path):
                 t, p = tmpl[name]
                 first[name] = np.array(o[: min(2048, p.shape[0]) * t.outputs]).reshape(-1, t.outputs)
         np.savez(keep_path, **first)
-    print(json.dumps(line))
+    print(json_line(line))
 
 
 def reference_gpu(kinds=("f64", "df64", "mixed"), steps=2, warmup=1, keep_path=None):
@@ -961,11 +975,11 @@ def main():
         cb = {"value": v, "unit": "points/s", "cores": os.cpu_count(), "kind": "port",
               "sample": "first 2048 points of each family per step (as the GPU arm's cpu_baseline), OpenMP over "
                         "all host cores, rates weighted by the families' shares"}
-        print(json.dumps({"impl": "reference", "metric": metric, "value": v, "unit": "points/s", "n_gpus": 1,
-                          "steps": args.steps, "warmup": args.warmup, "higher_is_better": True, "scaling": "weak",
-                          "vs_baseline": None, "dtype": "f64", "data": "synthetic", "config": config,
-                          "cpu_baseline": cb,
-                          "e2e": {"value": v, "unit": "points/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}))
+        print(json_line({"impl": "reference", "metric": metric, "value": v, "unit": "points/s", "n_gpus": 1,
+                         "steps": args.steps, "warmup": args.warmup, "higher_is_better": True, "scaling": "weak",
+                         "vs_baseline": None, "dtype": "f64", "data": "synthetic", "config": config,
+                         "cpu_baseline": cb,
+                         "e2e": {"value": v, "unit": "points/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}))
         return
 
     import torch
@@ -975,10 +989,10 @@ def main():
 
     build.build()
     if args.surrogate_kernels:
-        print(json.dumps({"surrogate_kernels": surrogate_kernels(torch)}))
+        print(json_line({"surrogate_kernels": surrogate_kernels(torch)}))
         return
     if args.listing:
-        print(json.dumps({"listing": listing_case(torch)}))
+        print(json_line({"listing": listing_case(torch)}))
         return
     if args.surrogate_only:
         kw = {}
@@ -990,7 +1004,7 @@ def main():
                 kw[key] = processes.PP4J if val == "pp4j" else processes.PP3J
                 continue
             kw[key] = float(val) if "." in val or "e" in val else int(val)
-        print(json.dumps({"surrogate": surrogate_line(torch, **kw)}))
+        print(json_line({"surrogate": surrogate_line(torch, **kw)}))
         return
     if world > 1:
         import datetime
@@ -1160,7 +1174,7 @@ def main():
         del batch
         dist.destroy_process_group()
     if rank == 0:
-        print(json.dumps(res))
+        print(json_line(res))
 
 
 def phase_space_major(p):
