@@ -22,10 +22,13 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 SOURCES = ["runner.cu", "batch.cu", "program.cpp", "schedule.cpp", "tiled_host.cu", "peak.cu", "stability.cu"]
 SG_SOURCES = ["surrogate.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+# Past 10 MB or so nvcc compresses a file's device code, and a process's first call of it waits for the
+# whole to be unpacked (the executor's: 7 of the first plan's 12 ms).
+PLAIN = ["--no-compress"]
 FLAGS = ["-O3", "-std=c++17", "-fmad=false", "-lineinfo", "-Xcompiler", "-fPIC", "-shared", "-cudart", "static",
-         "-Xptxas", "-warn-spills"] + ARCH
+         "-Xptxas", "-warn-spills"] + PLAIN + ARCH
 SG_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-shared", "-cudart", "static",
-            "-Xptxas", "-warn-spills"] + ARCH
+            "-Xptxas", "-warn-spills"] + PLAIN + ARCH
 
 RUNNER_DEPS = ["runner.cu", "batch.cu", "program.cpp", "program.h", "schedule.cpp", "schedule.h", "tiled_host.cu",
                "tiled_host.h", "peak.cu", "arith.cuh", "executor.cuh", "tiled.cuh", "tiled_fma.cu", "stability.cu"]

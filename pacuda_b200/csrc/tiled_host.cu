@@ -1,7 +1,10 @@
 // Host helpers of the on-chip executor (tiled_host.h).
 #include <stdio.h>
+#include <string.h>
 
 #include <algorithm>
+#include <utility>
+#include <vector>
 
 #include "../../include/pacman_recurrence.h"
 #include "../../include/pacuda_b200.h"
@@ -11,11 +14,31 @@
 namespace pacuda {
 
 namespace {
-template <class T> bool put(T **dst, const std::vector<T> &v, cudaStream_t s) {
-    size_t bytes = std::max<size_t>(1, v.size()) * sizeof(T);
-    if (cudaMalloc((void **)dst, bytes) != cudaSuccess) return false;
-    return v.empty() || cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s) == cudaSuccess;
-}
+
+// The arrays of a device plan, in one allocation and one copy (each of a plan's first call's several
+// allocations and copies waits for the driver).
+struct Slab {
+    std::vector<uint8_t> bytes;
+    std::vector<std::pair<void **, size_t>> arrays;
+    // room for `n` values that *dst is to point at, filled from `src` where there is one
+    template <class T> void add(T **dst, const T *src, size_t n) {
+        const size_t at = (bytes.size() + 255) / 256 * 256;
+        bytes.resize(at + std::max<size_t>(1, n) * sizeof(T));
+        if (src && n) memcpy(bytes.data() + at, src, n * sizeof(T));
+        arrays.push_back({(void **)dst, at});
+    }
+    template <class T> void add(T **dst, const std::vector<T> &v) { add(dst, v.data(), v.size()); }
+    // (waits for the copy)
+    bool upload(void **slab, cudaStream_t s) {
+        if (cudaMalloc(slab, bytes.size()) != cudaSuccess) {
+            *slab = nullptr;
+            return false;
+        }
+        for (auto &a : arrays) *a.first = (uint8_t *)*slab + a.second;
+        return cudaMemcpyAsync(*slab, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, s) == cudaSuccess &&
+               cudaStreamSynchronize(s) == cudaSuccess;
+    }
+};
 
 }  // namespace
 
@@ -42,14 +65,8 @@ const void *kernel_for(int kernel, bool abi = false) {
 }  // namespace
 
 void TiledDevice::release() {
-    cudaFree(ins);
-    cudaFree(loads);
-    cudaFree(amp_planes);
-    cudaFree(orders);
-    cudaFree(level_firsts);
-    cudaFree(entries);
-    cudaFree(recip_forms);
-    cudaFree(folded);
+    cudaFree(slab);
+    slab = nullptr;
     ins = nullptr;
     loads = amp_planes = orders = level_firsts = entries = recip_forms = nullptr;
     folded = nullptr;
@@ -102,9 +119,6 @@ bool upload_schedule(TiledDevice &t, uint32_t forms, int kernel, int threads, co
     // fetched (not run) ahead of a task's end, and beside the positions without a task
     const uint32_t padding = (uint32_t)packed.size();
     packed.resize(packed.size() + 8, make_uint4(0, 0, 0, 0));
-    t.ok = threads > 0 && put(&t.ins, packed, s) && put(&t.loads, t.host.loads, s) && put(&t.amp_planes, t.host.amp_planes, s) &&
-           put(&t.entries, folds.entries, s) && put(&t.recip_forms, folds.reciprocals, s) &&
-           cudaMalloc(&t.folded, std::max<size_t>(1, t.entry_count) * 16) == cudaSuccess;
     t.levels = (uint32_t)t.host.level_first.size() - 1;
     t.threads = threads;
     std::vector<uint32_t> first, firsts;
@@ -112,7 +126,7 @@ bool upload_schedule(TiledDevice &t, uint32_t forms, int kernel, int threads, co
     // tiled_lanes(P, tiled_block_threads(threads, b)) lanes, and many pairs give the same count
     std::vector<bool> made(kMaxLanes + 1, false);
     for (int b : kBlockChoices)
-        for (uint32_t np = 1; t.ok && np <= kMaxPoints; np++) {
+        for (uint32_t np = 1; threads > 0 && np <= kMaxPoints; np++) {
             uint32_t lanes = tiled_lanes(np, tiled_block_threads(threads, b));
             if (lanes == 0 || lanes > kMaxLanes || made[lanes]) continue;
             made[lanes] = true;
@@ -126,9 +140,16 @@ bool upload_schedule(TiledDevice &t, uint32_t forms, int kernel, int threads, co
         }
     // the executor fetches two positions of a lane ahead: up to two lane counts past the last one
     first.insert(first.end(), 3 * kMaxLanes, kNoTask | padding);
-    t.ok = t.ok && put(&t.orders, first, s) && put(&t.level_firsts, firsts, s);
-    // the host vectors must outlive the asynchronous copies
-    cudaStreamSynchronize(s);
+    Slab slab;
+    slab.add(&t.ins, packed);
+    slab.add(&t.loads, t.host.loads);
+    slab.add(&t.amp_planes, t.host.amp_planes);
+    slab.add(&t.entries, folds.entries);
+    slab.add(&t.recip_forms, folds.reciprocals);
+    slab.add(&t.orders, first);
+    slab.add(&t.level_firsts, firsts);
+    slab.add((uint4 **)&t.folded, (const uint4 *)nullptr, t.entry_count);  // (16 bytes an entry)
+    t.ok = threads > 0 && slab.upload(&t.slab, s);
     return t.ok;
 }
 

@@ -39,6 +39,7 @@ struct TiledDevice {
     // the folded constants' entries (schedule.h Folds) and values, the reciprocals' forms
     uint32_t *entries = nullptr, *recip_forms = nullptr;
     void *folded = nullptr;
+    void *slab = nullptr;  // one allocation for all of them
     uint32_t entry_count = 0, recips = 0;
     // per lane count G (of every blocks-per-SM choice and points per block): the lane order for G
     // lanes and its level boundaries, concatenated (offsets in 32-bit words, index G)
