@@ -48,8 +48,8 @@ struct pacuda_b200_plan {
     double *coefficients = nullptr;
     uint32_t *red_offsets = nullptr, *red_slots = nullptr;
     double *red_weights = nullptr;
-    uint32_t points = 1;      // points per block (a point has the block's threads / points lanes)
-    size_t point_bytes = 0;
+    // its points' bytes and points per block (a point has the block's threads / points lanes)
+    PlanSize size;
     bool fixed = false;
     bool wide = false;  // a level has more tasks than a point's default lanes
 };
@@ -90,9 +90,14 @@ struct pacuda_b200_batch {
 
 namespace {
 
-void fill_plan(const pacuda_b200_plan *p, TiledPlan &d, uint32_t points, size_t const_bytes, int blocks = 1) {
+// the bytes of the shape's points in a block
+size_t shape_bytes(const pacuda_b200_plan *p, const PlanShape &shape) {
+    return shape.points * (shape.keep ? p->size.kept : p->size.bare);
+}
+
+void fill_plan(const pacuda_b200_plan *p, TiledPlan &d, const PlanShape &shape, size_t const_bytes, int blocks = 1) {
     memset(&d, 0, sizeof d);
-    describe(p->tiled, p->forms, points, p->point_bytes, const_bytes, d, blocks);
+    describe(p->tiled, p->forms, shape, shape_bytes(p, shape) / shape.points, const_bytes, d, blocks);
     d.s64 = p->consts;
     d.f64 = p->consts + 2 * p->scales;
     d.factors = p->factors;
@@ -121,22 +126,7 @@ Offsets layout(size_t n) {
 }
 
 // blocks per SM chosen without timing (tiled_auto_blocks)
-int auto_blocks(const pacuda_b200_plan *p) {
-    return tiled_auto_blocks(p->kernel, p->point_bytes, tiled_const_bytes(p->tiled));
-}
-
-// The shared memory that the blocks of a launch keep for its plans' folded entries: the largest
-// table, or none (the entries are then read from global memory) where a plan's point would not fit
-// beside it. `which`: the launch's plans among `plans` (null: the first n).
-size_t group_const_bytes(pacuda_b200_plan *const *plans, const uint32_t *which, size_t n, int kernel, int blocks) {
-    size_t table = 0, point = 0;
-    for (size_t j = 0; j < n; j++) {
-        const pacuda_b200_plan *p = plans[which ? which[j] : j];
-        table = std::max(table, tiled_const_bytes(p->tiled));
-        point = std::max(point, p->point_bytes);
-    }
-    return table + point <= tiled_max_smem(kernel, blocks) ? table : 0;
-}
+int auto_blocks(const pacuda_b200_plan *p) { return tiled_auto_blocks(p->kernel, p->size); }
 
 // Few points: a batch that has no more points, in all its plans, than the GPU has SMs can run one
 // point per block and one block per SM, in one launch: each point has an SM and all its warps to
@@ -201,25 +191,25 @@ bool prepare(pacuda_b200_batch *b) {
         TiledPlan *plans = (TiledPlan *)(base + o.plans);
         unsigned long long *items = (unsigned long long *)(base + o.items);
         g.threads = tiled_threads(kernel, g.blocks);
-        g.const_bytes = group_const_bytes(b->plans.data(), g.plans.data(), m, kernel, g.blocks);
-        const size_t max_smem = tiled_max_smem(kernel, g.blocks) - g.const_bytes;
+        std::vector<PlanSize> sizes;
+        for (uint32_t k : g.plans) sizes.push_back(b->plans[k]->size);
+        std::vector<PlanShape> shapes;
+        // (each plan's choice where it fits this launch, else the default for it)
+        bool fits = launch_shapes(sizes, g.threads, tiled_max_smem(kernel, g.blocks), few, g.const_bytes, shapes);
         g.smem = 0;
         items[0] = 0;
         for (size_t j = 0; j < m; j++) {
-            const uint32_t k = g.plans[j];
-            pacuda_b200_plan *p = b->plans[k];
-            uint32_t most = tiled_max_points(p->point_bytes, g.threads, max_smem);
-            if (!most || p->tiled.threads != tiled_threads(kernel)) {
+            uint32_t k = g.plans[j];
+            const pacuda_b200_plan *p = b->plans[k];
+            fits = fits && tiled_block_threads(p->tiled.threads, g.blocks) == g.threads;
+            if (!fits) {
                 fprintf(stderr, "%s: a plan's point does not fit a block's shared memory\n", kTag);
                 return false;
             }
-            // the plan's choice where it fits this launch, else the default for it
-            uint32_t per = few ? 1 : tiled_points_fit(p->points, p->point_bytes, g.threads, max_smem)
-                               ? p->points
-                               : tiled_default_points(p->point_bytes, g.threads, max_smem);
+            const uint32_t per = shapes[j].points;
             b->points[k] = per;
-            fill_plan(p, plans[j], per, g.const_bytes, g.blocks);
-            g.smem = std::max<size_t>(g.smem, (size_t)per * p->point_bytes);
+            fill_plan(p, plans[j], shapes[j], g.const_bytes, g.blocks);
+            g.smem = std::max<size_t>(g.smem, shape_bytes(p, shapes[j]));
             items[j + 1] = items[j] + (b->count[k] + per - 1) / per;
             ((const double **)(base + o.external))[j] = b->external[k];
             ((double **)(base + o.output))[j] = b->output[k];
@@ -270,16 +260,14 @@ int launch(pacuda_b200_batch *b, cudaStream_t s) {
     return PACMAN_RECURRENCE_OK;
 }
 
-// the shared memory a block has for one plan's points
-size_t point_smem(const pacuda_b200_plan *p) {
-    pacuda_b200_plan *one = const_cast<pacuda_b200_plan *>(p);
-    return tiled_max_smem(p->kernel) - group_const_bytes(&one, nullptr, 1, p->kernel, 1);
-}
-
 // the default points per block (tiled_default_points)
 uint32_t default_points(const pacuda_b200_plan *p) {
-    uint32_t np = tiled_default_points(p->point_bytes, tiled_threads(p->kernel), point_smem(p));
-    return np ? np : 1u;
+    PlanSize size = p->size;
+    size.points = 0;
+    size_t table = 0;
+    std::vector<PlanShape> shape;
+    return launch_shapes({size}, tiled_threads(p->kernel), tiled_max_smem(p->kernel), false, table, shape) ? shape[0].points
+                                                                                                          : 1u;
 }
 
 }  // namespace
@@ -361,7 +349,7 @@ extern "C" pacuda_b200_plan *pacuda_b200_plan_create(const pacman_recurrence_cal
               to_device(&p->coefficients, c->term_coefficients, c->term_count) &&
               to_device(&p->red_offsets, offsets, (size_t)outputs + 1) &&
               to_device(&p->red_slots, slots.data(), slots.size()) &&
-              to_device(&p->red_weights, weights, offsets[outputs]) && upload_schedule(p->tiled, forms, p->kernel, tiled_threads(p->kernel), {c->scale_re, c->scale_im, c->factor_re, c->factor_im}, 0) &&
+              to_device(&p->red_weights, weights, offsets[outputs]) && upload_schedule(p->tiled, tiled_threads(p->kernel), {c->scale_re, c->scale_im, c->factor_re, c->factor_im}, 0) &&
               fold_values(p->tiled, p->kernel, p->consts + nc, p->scales, p->factors, 0) &&
               !failed(cudaDeviceSynchronize(), "plan upload");
     if (!ok) {
@@ -369,11 +357,13 @@ extern "C" pacuda_b200_plan *pacuda_b200_plan_create(const pacman_recurrence_cal
         pacuda_b200_plan_destroy(p);
         return nullptr;
     }
-    p->point_bytes = tiled_point_bytes(p->tiled, forms, p->kernel);
-    p->points = default_points(p);
+    p->size.kept = tiled_point_bytes(p->tiled, forms, p->kernel, true);
+    p->size.bare = tiled_point_bytes(p->tiled, forms, p->kernel, false);
+    p->size.table = tiled_const_bytes(p->tiled);
+    p->size.points = default_points(p);
     const std::vector<uint32_t> &first = p->tiled.host.level_first;
     for (size_t l = 0; l + 1 < first.size(); l++)
-        p->wide = p->wide || first[l + 1] - first[l] > tiled_lanes(p->points, tiled_threads(p->kernel));
+        p->wide = p->wide || first[l + 1] - first[l] > tiled_lanes(p->size.points, tiled_threads(p->kernel));
     return p;
 }
 
@@ -394,8 +384,8 @@ extern "C" uint64_t pacuda_b200_plan_flops(const pacuda_b200_plan *p) { return p
 extern "C" int pacuda_b200_plan_set_lanes_per_point(pacuda_b200_plan *p, uint32_t lanes) {
     if (!p) return PACMAN_RECURRENCE_INVALID;
     if (lanes == 0) {
-        p->fixed = false;
-        p->points = default_points(p);
+        p->fixed = p->size.chosen = false;
+        p->size.points = default_points(p);
         return PACMAN_RECURRENCE_OK;
     }
     int threads = tiled_threads(p->kernel);
@@ -403,14 +393,14 @@ extern "C" int pacuda_b200_plan_set_lanes_per_point(pacuda_b200_plan *p, uint32_
     uint32_t points = 0;
     for (uint32_t np = 1; np <= kMaxPoints; np++)
         if (tiled_lanes(np, threads) >= lanes) points = np;
-    if (!tiled_points_fit(points, p->point_bytes, threads, point_smem(p))) return PACMAN_RECURRENCE_INVALID;
-    p->points = points;
-    p->fixed = true;
+    if (!tiled_points_fit(points, p->size.bare, threads, tiled_max_smem(p->kernel))) return PACMAN_RECURRENCE_INVALID;
+    p->size.points = points;
+    p->fixed = p->size.chosen = true;
     return PACMAN_RECURRENCE_OK;
 }
 
 extern "C" uint32_t pacuda_b200_plan_lanes_per_point(const pacuda_b200_plan *p) {
-    return p ? tiled_lanes(p->points, p->tiled.threads) : 0;
+    return p ? tiled_lanes(p->size.points, p->tiled.threads) : 0;
 }
 
 extern "C" pacuda_b200_batch *pacuda_b200_batch_create(pacuda_b200_plan *const *plans, uint32_t nplans,
@@ -508,8 +498,10 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
         pacuda_b200_plan *p = b->plans[k], *one[1] = {p};
         const double *ext[1] = {b->external[k]};
         double *out[1] = {b->output[k]};
-        uint32_t n = b->count[k], keep = p->points;
-        p->points = points;
+        uint32_t n = b->count[k];
+        const PlanSize keep = p->size;
+        p->size.points = points;
+        p->size.chosen = true;
         pacuda_b200_batch *tb = pacuda_b200_batch_create(one, 1, ext, &n, out);
         float ms = -1.0f;
         if (tb) {
@@ -528,7 +520,7 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
             if (!ok) ms = -1.0f;
             pacuda_b200_batch_destroy(tb);
         }
-        p->points = keep;
+        p->size = keep;
         return ms;
     };
     // per plan: its fastest points per block (from the most that fit down to half of them:
@@ -537,16 +529,17 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
     const int kernel = b->plans[0]->kernel;
     for (size_t k = 0; k < b->plans.size(); k++) {
         pacuda_b200_plan *p = b->plans[k];
-        size_t cb = tiled_const_bytes(p->tiled);
         float best = -1.0f;
-        uint32_t best_points = p->points;
+        uint32_t best_points = p->size.points;
         int best_blocks = 0;
         for (int blocks : kBlockChoices) {
             int threads = tiled_threads(kernel, blocks);
-            size_t room = tiled_max_smem(kernel, blocks);
-            uint32_t most = room > cb ? tiled_max_points(p->point_bytes, threads, room - cb) : 0;
+            // (with its reciprocals and table beside them, but for points that are given or that fit without alone)
+            const size_t room = tiled_max_smem(kernel, blocks), table = p->size.table;
+            uint32_t most = room > table ? tiled_max_points(p->size.kept, threads, room - table) : 0;
+            if (!most || p->fixed) most = tiled_max_points(p->size.bare, threads, room);
             for (uint32_t points = most; points >= 1 && 2 * points >= most; points--) {
-                if (p->fixed && points != p->points) continue;
+                if (p->fixed && points != p->size.points) continue;
                 float ms = time_plan(k, points, blocks);
                 if (ms >= 0.0f && (best < 0.0f || ms < best)) {
                     best = ms;
@@ -556,7 +549,8 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
             }
         }
         if (best >= 0.0f) {
-            p->points = best_points;
+            p->size.points = best_points;
+            p->size.chosen = true;
             b->plan_blocks[k] = best_blocks;
             b->given[k] = 0;  // (the choice is the tuner's now)
         }
@@ -811,27 +805,26 @@ extern "C" int pacuda_b200_run_static(pacuda_b200_plan *const *plans, uint32_t n
     // is not applied); the plans' own choices are not changed
     int kernel = plans[0]->kernel;
     int threads = tiled_threads(kernel);
-    // the shared memory a block may have, less the plan constants every block holds (checked
-    // before anything is queued)
+    // the shared memory a block may have (checked before anything is queued)
     const size_t room = tiled_max_smem(kernel);
     if (room == 0) return PACMAN_RECURRENCE_DEVICE_ERROR;
-    const size_t const_bytes = group_const_bytes(plans, nullptr, nplans, kernel, 1);
-    const size_t max_smem = room - const_bytes;
+    std::vector<PlanSize> sizes;
+    for (uint32_t k = 0; k < nplans; k++) sizes.push_back(plans[k]->size);
+    std::vector<PlanShape> shapes;
+    size_t const_bytes = 0;
+    bool fits = launch_shapes(sizes, threads, room, false, const_bytes, shapes);
     StaticBlock block;
     memset(&block, 0, sizeof block);
     size_t smem = 0;
     for (uint32_t k = 0; k < nplans; k++) {
         const pacuda_b200_plan *p = plans[k];
-        uint32_t most = tiled_max_points(p->point_bytes, threads, max_smem);
-        if (!most || p->tiled.threads != threads) {
+        if (!fits || p->tiled.threads != threads) {
             fprintf(stderr, "%s: run_static: a plan's point does not fit a block's shared memory\n", kTag);
             return PACMAN_RECURRENCE_INVALID;
         }
-        uint32_t per = tiled_points_fit(p->points, p->point_bytes, threads, max_smem)
-                           ? p->points
-                           : tiled_default_points(p->point_bytes, threads, max_smem);
-        fill_plan(p, block.plans[k], per, const_bytes);
-        smem = std::max<size_t>(smem, (size_t)per * p->point_bytes);
+        const uint32_t per = shapes[k].points;
+        fill_plan(p, block.plans[k], shapes[k], const_bytes);
+        smem = std::max<size_t>(smem, shape_bytes(p, shapes[k]));
         block.items[k + 1] = block.items[k] + (count[k] + per - 1) / per;
         block.external[k] = external[k];
         block.output[k] = output[k];

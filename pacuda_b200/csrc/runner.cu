@@ -373,25 +373,33 @@ int onchip_launch(DeviceProgram *prog, const pacman_recurrence_call *c, const Ru
     if (prog->tiled_state == 0) {
         prog->tiled_state = -1;
         if (build_schedule(prog->host, c->current_planes, c->amplitude_planes, prog->tiled.host) &&
-            upload_schedule(prog->tiled, forms, kernel, tiled_threads(kernel), TiledConstants(), dev.stream))
+            upload_schedule(prog->tiled, tiled_threads(kernel), TiledConstants(), dev.stream))
             prog->tiled_state = 1;
     }
     // the lanes per point: as configured, else the default points per block; one block per SM (the
     // arena write-back of a block's interleaved points is coalesced over them: several blocks of
     // fewer points measured 19 % slower for gg>ggg through this path)
     int threads = prog->tiled_state == 1 ? tiled_threads(kernel) : 0;
-    size_t pb = prog->tiled_state == 1 ? tiled_point_bytes(prog->tiled, forms, kernel) : 0;
-    size_t cb = tiled_const_bytes(prog->tiled);
-    if (cb + pb > (threads ? tiled_max_smem(kernel) : 0)) cb = 0;  // (the entries stay in global memory)
-    size_t room = threads ? tiled_max_smem(kernel) - cb : 0;
-    uint32_t np = threads && prog->tiled.threads == threads ? tiled_default_points(pb, threads, room) : 0;
-    if (np && current.lanes_per_point) {
-        uint32_t want = 0;  // the most points per block whose lanes are at least the configured count
-        for (uint32_t n = 1; n <= kMaxPoints; n++)
-            if (tiled_lanes(n, threads) >= current.lanes_per_point) want = n;
-        np = tiled_points_fit(want, pb, threads, room) ? want : 0;
+    PlanSize size;
+    if (threads) {
+        size.kept = tiled_point_bytes(prog->tiled, forms, kernel, true);
+        size.bare = tiled_point_bytes(prog->tiled, forms, kernel, false);
+        size.table = tiled_const_bytes(prog->tiled);
     }
+    if (current.lanes_per_point) {  // the most points per block whose lanes are at least the configured count
+        size.chosen = true;
+        for (uint32_t n = 1; n <= kMaxPoints; n++)
+            if (tiled_lanes(n, threads) >= current.lanes_per_point) size.points = n;
+    }
+    size_t cb = 0;
+    std::vector<PlanShape> shape;
+    uint32_t np = 0;
+    if (threads && prog->tiled.threads == threads && (!size.chosen || size.points) &&
+        launch_shapes({size}, threads, tiled_max_smem(kernel), false, cb, shape) &&
+        (!size.chosen || shape[0].points == size.points))
+        np = shape[0].points;
     if (!np) return current.executor == PACUDA_B200_EXECUTOR_ONCHIP ? 2 : 0;
+    const size_t pb = shape[0].keep ? size.kept : size.bare;
     size_t smem = cb + (size_t)np * pb;
     // descriptors: TiledPlan | item_first[2] | external[1] | count[1] | counter
     const size_t o_items = (sizeof(TiledPlan) + 15) / 16 * 16, o_ext = o_items + 16, o_count = o_ext + 8,
@@ -400,7 +408,7 @@ int onchip_launch(DeviceProgram *prog, const pacman_recurrence_call *c, const Ru
     if (!dev.launch_dev.reserve(total, "descriptors")) return -1;
     memset(dev.launch_host, 0, total);
     TiledPlan &p = *(TiledPlan *)dev.launch_host;
-    describe(prog->tiled, forms, np, pb, cb, p);
+    describe(prog->tiled, forms, shape[0], pb, cb, p);
     p.s64 = a.s64;
     p.f64 = a.f64;
     p.factors = a.factors;

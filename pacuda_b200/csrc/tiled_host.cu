@@ -3,7 +3,7 @@
 #include <string.h>
 
 #include <algorithm>
-#include <utility>
+#include <memory>
 #include <vector>
 
 #include "../../include/pacman_recurrence.h"
@@ -15,27 +15,36 @@ namespace pacuda {
 
 namespace {
 
-// The arrays of a device plan, in one allocation and one copy (each of a plan's first call's several
-// allocations and copies waits for the driver).
+// The arrays of a device plan, in one allocation and one copy (several of each were a few percent of a
+// small plan's first call).
 struct Slab {
-    std::vector<uint8_t> bytes;
-    std::vector<std::pair<void **, size_t>> arrays;
+    struct Array {
+        void **dst;
+        const void *src;
+        size_t at, bytes;
+    };
+    std::vector<Array> arrays;
+    size_t total = 0;
     // room for `n` values that *dst is to point at, filled from `src` where there is one
     template <class T> void add(T **dst, const T *src, size_t n) {
-        const size_t at = (bytes.size() + 255) / 256 * 256;
-        bytes.resize(at + std::max<size_t>(1, n) * sizeof(T));
-        if (src && n) memcpy(bytes.data() + at, src, n * sizeof(T));
-        arrays.push_back({(void **)dst, at});
+        arrays.push_back({(void **)dst, src, total, src ? n * sizeof(T) : 0});
+        total += (std::max<size_t>(1, n) * sizeof(T) + 255) / 256 * 256;
     }
     template <class T> void add(T **dst, const std::vector<T> &v) { add(dst, v.data(), v.size()); }
     // (waits for the copy)
     bool upload(void **slab, cudaStream_t s) {
-        if (cudaMalloc(slab, bytes.size()) != cudaSuccess) {
+        if (cudaMalloc(slab, total) != cudaSuccess) {
             *slab = nullptr;
             return false;
         }
-        for (auto &a : arrays) *a.first = (uint8_t *)*slab + a.second;
-        return cudaMemcpyAsync(*slab, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, s) == cudaSuccess &&
+        std::unique_ptr<uint8_t[]> host(new uint8_t[total]);
+        size_t end = 0;
+        for (const Array &a : arrays) {
+            *a.dst = (uint8_t *)*slab + a.at;
+            if (a.bytes) memcpy(host.get() + a.at, a.src, a.bytes);
+            if (a.bytes) end = a.at + a.bytes;
+        }
+        return cudaMemcpyAsync(*slab, host.get(), end, cudaMemcpyHostToDevice, s) == cudaSuccess &&
                cudaStreamSynchronize(s) == cudaSuccess;
     }
 };
@@ -67,7 +76,7 @@ const void *kernel_for(int kernel, bool abi = false) {
 void TiledDevice::release() {
     cudaFree(slab);
     slab = nullptr;
-    ins = nullptr;
+    ins = bare = nullptr;
     loads = amp_planes = orders = level_firsts = entries = recip_forms = nullptr;
     folded = nullptr;
     ok = false;
@@ -95,30 +104,28 @@ bool pack_ins(const Ins &i, bool end, uint4 &w) {
     return true;
 }
 
-bool upload_schedule(TiledDevice &t, uint32_t forms, int kernel, int threads, const TiledConstants &c, cudaStream_t s) {
+bool upload_schedule(TiledDevice &t, int threads, const TiledConstants &c, cudaStream_t s) {
     Folds folds;
     fold_constants(t.host, c.scale_re, c.scale_im, c.factor_re, c.factor_im, folds);
     t.entry_count = (uint32_t)folds.entries.size() / 2;
     t.recips = (uint32_t)folds.reciprocals.size();
-    if (tiled_const_bytes(t) + tiled_point_bytes(t, forms, kernel) > tiled_max_smem(kernel)) {
-        // (a point at the limit of the shared memory: its propagators keep computing theirs)
-        t.recips = 0;
-        folds.reciprocals.clear();
-        for (Ins &i : folds.ins)
-            if (ins_kind(i) == K_PROP) i.s = kNoReciprocal;
-    }
     std::vector<uint8_t> end(folds.ins.size(), 0);
     for (size_t k = 1; k < folds.task_first.size(); k++) end[folds.task_first[k] - 1] = 1;
-    std::vector<uint4> packed(folds.ins.size());
-    for (size_t n = 0; n < packed.size(); n++)
-        if (!pack_ins(folds.ins[n], end[n], packed[n])) {
+    std::vector<uint4> packed(folds.ins.size()), bare(folds.ins.size());
+    for (size_t n = 0; n < packed.size(); n++) {
+        Ins i = folds.ins[n];
+        bool ok = pack_ins(i, end[n], packed[n]);
+        if (ins_kind(i) == K_PROP) i.s = kNoReciprocal;
+        if (!ok || !pack_ins(i, end[n], bare[n])) {
             t.host.why = "an instruction's field does not fit the on-chip executor's 16-byte form";
             t.ok = false;
             return false;
         }
+    }
     // fetched (not run) ahead of a task's end, and beside the positions without a task
     const uint32_t padding = (uint32_t)packed.size();
     packed.resize(packed.size() + 8, make_uint4(0, 0, 0, 0));
+    bare.resize(packed.size(), make_uint4(0, 0, 0, 0));
     t.levels = (uint32_t)t.host.level_first.size() - 1;
     t.threads = threads;
     std::vector<uint32_t> first, firsts;
@@ -142,12 +149,13 @@ bool upload_schedule(TiledDevice &t, uint32_t forms, int kernel, int threads, co
     first.insert(first.end(), 3 * kMaxLanes, kNoTask | padding);
     Slab slab;
     slab.add(&t.ins, packed);
+    slab.add(&t.orders, first);
+    slab.add(&t.level_firsts, firsts);
     slab.add(&t.loads, t.host.loads);
     slab.add(&t.amp_planes, t.host.amp_planes);
     slab.add(&t.entries, folds.entries);
     slab.add(&t.recip_forms, folds.reciprocals);
-    slab.add(&t.orders, first);
-    slab.add(&t.level_firsts, firsts);
+    slab.add(&t.bare, bare);
     slab.add((uint4 **)&t.folded, (const uint4 *)nullptr, t.entry_count);  // (16 bytes an entry)
     t.ok = threads > 0 && slab.upload(&t.slab, s);
     return t.ok;
@@ -171,10 +179,11 @@ bool fold_values(const TiledDevice &t, int kernel, const void *constants, uint32
     return cudaGetLastError() == cudaSuccess;
 }
 
-size_t tiled_point_bytes(const TiledDevice &t, uint32_t forms, int kernel) {
+size_t tiled_point_bytes(const TiledDevice &t, uint32_t forms, int kernel, bool keep) {
     const Schedule &s = t.host;
+    const size_t recips = keep ? t.recips : 0;
     size_t value = kernel == PACMAN_RECURRENCE_KERNEL_MIXED || kernel == PACMAN_RECURRENCE_KERNEL_MIXED64 ? 4 : 8;
-    size_t per_point = 2 * value * s.cur_slots + 2 * 8 * s.amp_slots + 8 * ((size_t)s.terms + t.recips) + 8 * 4 * (size_t)forms;
+    size_t per_point = 2 * value * s.cur_slots + 2 * 8 * s.amp_slots + 8 * (s.terms + recips) + 8 * 4 * (size_t)forms;
     return (per_point + 15) / 16 * 16;
 }
 
@@ -211,43 +220,27 @@ size_t tiled_max_smem(int kernel, int blocks) {
     return limit > attr.sharedSizeBytes ? limit - attr.sharedSizeBytes : 0;
 }
 
-bool tiled_points_fit(uint32_t points, size_t point_bytes, int threads, size_t max_smem) {
-    return points >= 1 && points <= kMaxPoints && threads >= 32 && (size_t)points * point_bytes <= max_smem;
-}
-
-uint32_t tiled_max_points(size_t point_bytes, int threads, size_t max_smem) {
-    for (uint32_t np = kMaxPoints; np >= 1; np--)
-        if (tiled_points_fit(np, point_bytes, threads, max_smem)) return np;
-    return 0;
-}
-
-int tiled_auto_blocks(int kernel, size_t point_bytes, size_t const_bytes) {
-    auto most = [&](int blocks) {
-        size_t room = tiled_max_smem(kernel, blocks);
-        return room > const_bytes ? tiled_max_points(point_bytes, tiled_threads(kernel, blocks), room - const_bytes) : 0u;
+int tiled_auto_blocks(int kernel, const PlanSize &size) {
+    PlanSize plan = size;
+    plan.points = 0;
+    std::vector<PlanShape> shape;
+    size_t table = 0;
+    auto fits = [&](int blocks) {
+        return launch_shapes({plan}, tiled_threads(kernel, blocks), tiled_max_smem(kernel, blocks), false, table, shape);
     };
-    size_t room1 = tiled_max_smem(kernel, 1);
-    uint32_t one = room1 > const_bytes ? tiled_default_points(point_bytes, tiled_threads(kernel, 1), room1 - const_bytes) : 0;
+    uint32_t one = fits(1) ? shape[0].points : 0;
     // the choices to try, most blocks first
     static const int few[] = {4, 2};
     const int *first = one && one <= 4 ? few : few + 1;
     for (const int *b = first; b != few + 2; b++)
-        if (most(*b)) return *b;
+        if (fits(*b)) return *b;
     return 1;
 }
 
-uint32_t tiled_default_points(size_t point_bytes, int threads, size_t max_smem) {
-    uint32_t best = 0;
-    for (uint32_t np = 1; np <= kMaxPoints; np++)
-        if (tiled_points_fit(np, point_bytes, threads, max_smem) && (!best || np * (32 / np) >= best * (32 / best)))
-            best = np;
-    return best;
-}
-
-void describe(const TiledDevice &t, uint32_t forms, uint32_t points, size_t point_bytes, size_t const_bytes, TiledPlan &p,
-              int blocks) {
-    p.ins = t.ins;
-    const uint32_t lanes = tiled_lanes(points, tiled_block_threads(t.threads, blocks));
+void describe(const TiledDevice &t, uint32_t forms, const PlanShape &shape, size_t point_bytes, size_t const_bytes,
+              TiledPlan &p, int blocks) {
+    p.ins = shape.keep ? t.ins : t.bare;
+    const uint32_t lanes = tiled_lanes(shape.points, tiled_block_threads(t.threads, blocks));
     p.order = t.orders + t.order_at[lanes];
     p.level_first = t.level_firsts + t.level_at[lanes];
     p.levels = t.levels;
@@ -255,7 +248,7 @@ void describe(const TiledDevice &t, uint32_t forms, uint32_t points, size_t poin
     p.amp_slots = t.host.amp_slots;
     p.terms = t.host.terms;
     p.forms = forms;
-    p.points = points;
+    p.points = shape.points;
     p.lanes = lanes;
     p.point_bytes = (uint32_t)point_bytes;
     p.loads = t.loads;
@@ -265,7 +258,7 @@ void describe(const TiledDevice &t, uint32_t forms, uint32_t points, size_t poin
     p.entries = t.entry_count;
     p.near = 16 * (size_t)t.entry_count <= const_bytes ? t.entry_count : 0;
     p.recip_forms = t.recip_forms;
-    p.recips = t.recips;
+    p.recips = shape.keep ? t.recips : 0;
 }
 
 bool launch_tiled(int kernel, const TiledLaunch &args, int threads, size_t smem, int grid, cudaStream_t stream) {

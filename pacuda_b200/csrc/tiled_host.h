@@ -5,15 +5,13 @@
 #include <stdint.h>
 
 #include "schedule.h"
+#include "shapes.h"
 
 namespace pacuda {
 
 struct TiledPlan;
 struct TiledLaunch;
 
-// points per block: 1 .. kMaxPoints; a point then has warps * floor(32 / P) lanes (a lane of all
-// P points is P adjacent threads of one warp)
-constexpr uint32_t kMaxPoints = 32;
 // blocks per SM: 1 (one block of all the warps the registers allow) or several independent blocks
 // that share those warps and reach their barriers at different times; a block of b per SM has
 // floor(warps / b) warps, so 3 and 5 leave one warp unused (16 warps: 5 x 3 = 15)
@@ -34,7 +32,8 @@ constexpr uint32_t kMaxLanes = 512;
 
 struct TiledDevice {
     Schedule host;
-    uint4 *ins = nullptr;  // the schedule's instructions, packed (pack_ins)
+    uint4 *ins = nullptr;   // the schedule's instructions, packed (pack_ins)
+    uint4 *bare = nullptr;  // the same for points that keep no reciprocals: each propagator computes its own
     uint32_t *loads = nullptr, *amp_planes = nullptr;
     // the folded constants' entries (schedule.h Folds) and values, the reciprocals' forms
     uint32_t *entries = nullptr, *recip_forms = nullptr;
@@ -65,42 +64,33 @@ struct TiledConstants {
     const double *scale_re = nullptr, *scale_im = nullptr, *factor_re = nullptr, *factor_im = nullptr;
 };
 // the schedule's arrays on the device, with the lane orders of every points-per-block count for
-// blocks of `threads` of kernel kind `kernel`; false (with the reason in t.host.why) when an
-// instruction does not pack. A point keeps its reciprocals where one point still fits a block with
-// them, else (none kept) each propagator computes its own.
-bool upload_schedule(TiledDevice &t, uint32_t forms, int kernel, int threads, const TiledConstants &c, cudaStream_t stream);
+// blocks of `threads`; false (with the reason in t.host.why) when an instruction does not pack
+bool upload_schedule(TiledDevice &t, int threads, const TiledConstants &c, cudaStream_t stream);
 // fills t.folded from the constants in the kind's layout (device: scales re, im, factors re, im)
 bool fold_values(const TiledDevice &t, int kernel, const void *constants, uint32_t scales, uint32_t factors,
                  cudaStream_t stream);
 
-// bytes of shared memory one point needs (kernel: PACMAN_RECURRENCE_KERNEL_*), 16-aligned
-size_t tiled_point_bytes(const TiledDevice &t, uint32_t forms, int kernel);
+// bytes of shared memory one point needs (kernel: PACMAN_RECURRENCE_KERNEL_*), 16-aligned, with its
+// reciprocals or without
+size_t tiled_point_bytes(const TiledDevice &t, uint32_t forms, int kernel, bool keep);
 
 // a block's threads with `blocks` blocks per SM (as the kernel's registers allow, at most 512 per
 // SM) and its largest dynamic shared memory
 int tiled_threads(int kernel, int blocks = 1);
 size_t tiled_max_smem(int kernel, int blocks = 1);
 
-// whether a block of `threads` runs `points` points within `max_smem` bytes
-bool tiled_points_fit(uint32_t points, size_t point_bytes, int threads, size_t max_smem);
-// the most points per block that fit, or 0
-uint32_t tiled_max_points(size_t point_bytes, int threads, size_t max_smem);
-// Blocks per SM chosen without timing for points of `point_bytes` and constants of `const_bytes`:
+// Blocks per SM chosen without timing:
 // four (their points run on fewer, independent warps: 4 each) when at most four points fit a
 // block of all the warps, else two; fewer when the points do not fit. (Measured on B200: gg>ggg,
 // 4 points per 16 warps, gains 5 % at four blocks over two; five blocks' shared memory leaves L1
 // too little room for its instruction stream since the spread slot layout; qg>qgg, 16 points,
 // loses 14 % at four.)
-int tiled_auto_blocks(int kernel, size_t point_bytes, size_t const_bytes);
+int tiled_auto_blocks(int kernel, const PlanSize &size);
 
-// the default points per block: of those that fit, the count that leaves the fewest threads of a
-// warp without a lane (P * floor(32 / P) largest), the larger on ties; 0 when none fits
-uint32_t tiled_default_points(size_t point_bytes, int threads, size_t max_smem);
-
-// fills the schedule fields of a plan descriptor for `points` points per block, `blocks` per SM
-// with `const_bytes` of the block's shared memory for folded entries
-void describe(const TiledDevice &t, uint32_t forms, uint32_t points, size_t point_bytes, size_t const_bytes, TiledPlan &p,
-              int blocks = 1);
+// fills the schedule fields of a plan descriptor for a shape in a launch of `blocks` per SM with
+// `const_bytes` of the block's shared memory for folded entries
+void describe(const TiledDevice &t, uint32_t forms, const PlanShape &shape, size_t point_bytes, size_t const_bytes,
+              TiledPlan &p, int blocks = 1);
 
 // launches the persistent kernel (`grid` blocks: the SMs times the blocks per SM) with `smem` bytes
 // of shared memory
