@@ -333,10 +333,14 @@ __device__ __forceinline__ void final32(const float (&u)[Space<4>::NUMBERS], dou
 
 // What the f32 partons p say of a candidate's cuts (see above). The margins hold both ways: a value
 // beyond the cut by more than its error is beyond it in f64, on either side. (Comparisons are written
-// so that a NaN is not sure of anything; past 1e18 the squares of f32 overflow.)
+// so that a NaN is not sure of anything. The error is a share of sqrt(s) only where f32's products neither
+// underflow nor overflow. The largest is boost32's q q par, up to s^1.5 / 8; below 1e-11 its last bit, 1e-45,
+// over (e + m) m >= 3e-4 s is no longer far under 5e-7 sqrt(s), above 1e13 it overflows. Outside 1e-9 to 1e12
+// the f64 cuts decide every candidate.)
 enum Look : uint32_t { LOOK_FAILS, LOOK_PASSES, LOOK_UNSURE };
 template <int F>
 __device__ __forceinline__ Look look32(const float (&p)[F][3], double sqrt_s, const Cuts &c) {
+    if (!(sqrt_s >= 1e-9 && sqrt_s <= 1e12)) return LOOK_UNSURE;
     const float d = PHASE32_DELTA * (float)sqrt_s, sh = sinhf((float)c.eta_max), dz = d * (1.0f + 1.5f * sh);
     bool sure = true;
     float pt[F];
@@ -351,7 +355,7 @@ __device__ __forceinline__ Look look32(const float (&p)[F][3], double sqrt_s, co
     float eta[F], phi[F], err[F];
     for (int i = 0; i < F; i++) {
         const float low = pt[i] - 2.0f * d;
-        if (!(low > 0.0f) || !(pt[i] < 1e18f)) return LOOK_UNSURE;
+        if (!(low > 0.0f)) return LOOK_UNSURE;
         const float z = p[i][2] / pt[i];
         eta[i] = copysignf(__logf(fabsf(z) + sqrtf(z * z + 1.0f)), z);
         phi[i] = atan2f(p[i][1], p[i][0]);
