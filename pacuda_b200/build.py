@@ -32,7 +32,7 @@ SG_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-shared", 
 
 RUNNER_DEPS = ["runner.cu", "batch.cu", "program.cpp", "program.h", "schedule.cpp", "schedule.h", "tiled_host.cu",
                "tiled_host.h", "peak.cu", "arith.cuh", "executor.cuh", "tiled.cuh", "tiled_fma.cu", "stability.cu", "shapes.h"]
-SG_DEPS = ["surrogate.cu", "umma.cuh"]
+SG_DEPS = ["surrogate.cu", "umma.cuh", "phase.cuh"]
 
 
 def _stale(target, deps, headers):
