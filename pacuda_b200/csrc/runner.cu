@@ -351,6 +351,7 @@ const DeviceProgram *prepare(const pacman_recurrence_call *c, int *status) {
     if (dev.scratch.ins) {
         cudaStreamSynchronize(dev.stream);
         cudaFree(dev.scratch.ins);
+        dev.scratch.tiled.release();
     }
     dev.scratch = std::move(p);
     return &dev.scratch;
