@@ -19,7 +19,7 @@ INCLUDE = os.path.join(HERE, "..", "include")
 LIB = os.path.join(HERE, "librecurrence.so")
 SG_LIB = os.path.join(HERE, "libsurrogate.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-SOURCES = ["runner.cu", "batch.cu", "program.cpp", "schedule.cpp", "tiled_host.cu", "peak.cu", "stability.cu"]
+SOURCES = ["runner.cu", "batch.cu", "program.cpp", "schedule.cpp", "tiled_host.cu", "tiled_far.cu", "peak.cu", "stability.cu"]
 SG_SOURCES = ["surrogate.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # Past 10 MB or so nvcc compresses a file's device code, and a process's first call of it waits for the
@@ -31,7 +31,8 @@ SG_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-shared", 
             "-Xptxas", "-warn-spills"] + PLAIN + ARCH
 
 RUNNER_DEPS = ["runner.cu", "batch.cu", "program.cpp", "program.h", "schedule.cpp", "schedule.h", "tiled_host.cu",
-               "tiled_host.h", "peak.cu", "arith.cuh", "executor.cuh", "tiled.cuh", "tiled_fma.cu", "stability.cu", "shapes.h"]
+               "tiled_host.h", "peak.cu", "arith.cuh", "executor.cuh", "tiled.cuh", "tiled_fma.cu", "tiled_far.cu", "stability.cu",
+               "shapes.h"]
 SG_DEPS = ["surrogate.cu", "umma.cuh", "phase.cuh"]
 
 

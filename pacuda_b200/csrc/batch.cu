@@ -59,6 +59,7 @@ struct LaunchGroup {
     std::vector<uint32_t> plans;  // indices into the batch's plans
     int blocks = 1, threads = 0;
     size_t smem = 0, const_bytes = 0;
+    bool far = false;             // a plan needs the kernels for large tables
     size_t at = 0;                // its section of the descriptor block
 };
 
@@ -210,6 +211,7 @@ bool prepare(pacuda_b200_batch *b) {
             b->points[k] = per;
             fill_plan(p, plans[j], shapes[j], g.const_bytes, g.blocks);
             g.smem = std::max<size_t>(g.smem, shape_bytes(p, shapes[j]));
+            g.far = g.far || tiled_far(p->tiled);
             items[j + 1] = items[j] + (b->count[k] + per - 1) / per;
             ((const double **)(base + o.external))[j] = b->external[k];
             ((double **)(base + o.output))[j] = b->output[k];
@@ -235,6 +237,7 @@ TiledLaunch launch_args(const pacuda_b200_batch *b, const LaunchGroup &g) {
     L.counter = (unsigned long long *)(base + o.counter);
     L.abi = false;
     L.const_bytes = (uint32_t)g.const_bytes;
+    L.far = g.far;
     return L;
 }
 
@@ -846,6 +849,7 @@ extern "C" int pacuda_b200_run_static(pacuda_b200_plan *const *plans, uint32_t n
     L.counter = (unsigned long long *)(scratch + kStaticCounter);
     L.abi = false;
     L.const_bytes = (uint32_t)const_bytes;
+    for (uint32_t k = 0; k < nplans; k++) L.far = L.far || tiled_far(plans[k]->tiled);
     if (!launch_tiled(kernel, L, threads, smem, device_sms(), s) || failed(cudaGetLastError(), "run_static launch"))
         return PACMAN_RECURRENCE_DEVICE_ERROR;
     return PACMAN_RECURRENCE_OK;

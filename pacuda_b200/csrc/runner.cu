@@ -445,6 +445,7 @@ int onchip_launch(DeviceProgram *prog, const pacman_recurrence_call *c, const Ru
     L.mom = forms_on_device ? nullptr : a.mom;
     L.ld = a.ld;
     L.const_bytes = (uint32_t)cb;
+    L.far = tiled_far(prog->tiled);
     // (a table that stays in global memory is folded here, for this call's constants)
     if ((!cb && !fold_values(prog->tiled, kernel, a.kconst, a.scales, a.factors, dev.stream)) ||
         !launch_tiled(kernel, L, threads, smem, dev.sms, dev.stream) || failed(cudaGetLastError(), "launch")) return -1;

@@ -76,11 +76,14 @@ struct TiledLaunch {
     const double *mom;                     // uploaded forms (f64 planes), or null
     size_t ld;
     uint32_t const_bytes;                  // shared memory kept for a plan's folded entries
+    bool far;                              // a plan has more entries than 16 bits index
 };
 
 // The on-chip executor's 16-byte instruction: a head, the forms' bytes, then (a, b), (c, s), (x, y)
 // as 16-bit pairs. Every field of a plan whose points fit shared memory fits (slots and constant
-// indices below 65536, forms below 256); the host checks. The head's sixteen bits:
+// indices below 65536, forms below 256); the host checks. An entry's index, which a plan with many pairs
+// of constants may need more bits for, has its upper half in a field that its row does not use. The
+// head's sixteen bits:
 constexpr uint32_t H_CODE = 15;        // RowCode
 constexpr uint32_t H_CLASS = 3 << 4;   // FoldClass
 constexpr uint32_t H_END = 1 << 6;     // the task's last instruction
@@ -104,6 +107,10 @@ struct Row16 {
     __device__ __forceinline__ uint32_t s() const { return w.z >> 16; }
     __device__ __forceinline__ uint32_t x() const { return w.w & 0xffff; }
     __device__ __forceinline__ uint32_t y() const { return w.w >> 16; }
+    // the entry of a contribution (s, x), a propagator or identity (x, c), a closure's first (y, x)
+    __device__ __forceinline__ uint32_t entry_s() const { return __byte_perm(w.z, w.w, 0x5432); }
+    __device__ __forceinline__ uint32_t entry_x() const { return __byte_perm(w.w, w.z, 0x5410); }
+    __device__ __forceinline__ uint32_t entry_y() const { return __byte_perm(w.w, 0, 0x1032); }
 };
 
 // a hint: the line holding `p` into L1 (no register waits for it)
@@ -140,8 +147,9 @@ struct AbiItem {
 static __shared__ AbiItem abi_item;
 
 // NP: the block's points when known at compile time (0: np at run time); with NP a slot's
-// address is a shift of its index and its components' addresses constant offsets from it
-template <class K, bool ABI, int NP = 0> struct SlotView {
+// address is a shift of its index and its components' addresses constant offsets from it.
+// FAR: a table of more entries than 16 bits index
+template <class K, bool ABI, int NP = 0, bool FAR = false> struct SlotView {
     typedef typename K::R R;
     typedef typename K::Den Den;
     typedef typename K::Amp Amp;
@@ -154,6 +162,10 @@ template <class K, bool ABI, int NP = 0> struct SlotView {
     const Pair<R> *folded_;  // the plan's folded entries (in shared memory where NP is known)
     uint32_t np, pw;      // the block's points (interleaved) and this thread's
     static constexpr int kPoints = NP;
+    // a row's entry
+    __device__ __forceinline__ uint32_t entry_s(const Row16 &o) const { return FAR ? o.entry_s() : o.s(); }
+    __device__ __forceinline__ uint32_t entry_x(const Row16 &o) const { return FAR ? o.entry_x() : o.x(); }
+    __device__ __forceinline__ uint32_t entry_y(const Row16 &o) const { return FAR ? o.entry_y() : o.y(); }
     __device__ __forceinline__ uint32_t at(uint32_t slot) const { return NP ? slot * NP + pw : slot * np + pw; }
     // the same view with the addressing of N points per block (valid when np == N)
     // and its entries at `near` in shared memory
@@ -272,7 +284,7 @@ __device__ __forceinline__ void tile_contribution(const V &v, const Row16 &o, Cx
     Cx<R> l[c0], r[c1], val[cd], scale = cx(konst<R>(1.0), konst<R>(0.0));
     R q0[4], q1[4];
     const uint32_t a = o.a(), b = o.b();
-    if (CLS != (int)C_ONE) scale = v.folded(o.s());
+    if (CLS != (int)C_ONE) scale = v.folded(v.entry_s(o));
 #pragma unroll
     for (int k = 0; k < c0; k++) l[k] = v.cur(a + k);
 #pragma unroll
@@ -329,7 +341,7 @@ __device__ __forceinline__ void tile_propagator(const V &v, const Row16 &o) {
         v.form(o.f0(), q);
         reciprocal = form_reciprocal<K>(q);
     }
-    const Cx<R> s = scaled(v.folded(o.x()), reciprocal);
+    const Cx<R> s = scaled(v.folded(v.entry_x(o)), reciprocal);
     Cx<R> c[m], out[m];
 #pragma unroll
     for (int k = 0; k < m; k++) out[k] = v.cur(a + k);
@@ -362,7 +374,7 @@ __device__ __forceinline__ void tile_propagator(const V &v, const Row16 &o) {
 template <class K, class V> __device__ __forceinline__ void tile_vector_propagator(const V &v, const Row16 &o) {
     typedef typename K::R R;
     const uint32_t a = o.a();
-    const R s = v.folded(o.x()).im * v.reciprocal(o.s());
+    const R s = v.folded(v.entry_x(o)).im * v.reciprocal(o.s());
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const Cx<R> c = v.cur(a + k);
@@ -388,7 +400,7 @@ template <class K, int N, class V>
 __device__ __forceinline__ void tile_closure_term(const V &v, const Row16 &o, const Cx<typename K::R> *acc) {
     typedef typename K::Amp Amp;
     Amp dr = konst<Amp>(0.0), di = konst<Amp>(0.0);
-    const uint32_t b = o.b(), y = o.y();
+    const uint32_t b = o.b(), y = v.entry_y(o);
 #pragma unroll
     for (int k = 0; k < N; k++) add_closure<true>(acc[k], v.cur(b + k), v.folded(y + k), dr, di);
     v.put_term(o.c(), dr, di);
@@ -405,7 +417,7 @@ __device__ __forceinline__ void tile_closure(const V &v, const Row16 &o, const C
     } else {
         v.amp(o.c(), dr, di);
     }
-    const uint32_t a = o.a(), b = o.b(), n = o.s(), y = o.y();
+    const uint32_t a = o.a(), b = o.b(), n = o.s(), y = v.entry_y(o);
     if (o.w.x & H_ACC0) {
         // parent 0 is the task's sums (at most 6 components): indices known at compile time keep
         // the sums in registers
@@ -424,7 +436,7 @@ __device__ __forceinline__ void tile_closure(const V &v, const Row16 &o, const C
 // identity (op 10) and clear (op 1) over `b` components
 template <class K, class V> __device__ __forceinline__ void tile_identity(const V &v, const Row16 &o) {
     typedef typename K::R R;
-    const Cx<R> f = v.folded(o.x());
+    const Cx<R> f = v.folded(v.entry_x(o));
     for (uint32_t k = 0; k < o.b(); k++) {
         Cx<R> x = times_factor(f.re, f.im, v.cur(o.a() + k));
         v.put(o.a() + k, x);
@@ -614,8 +626,10 @@ __device__ __forceinline__ void run_levels(const V &v, const TiledPlan &p, doubl
     }
 }
 
-// ABI: the C ABI's mode (arena in and out) or a batch's (outputs only)
-template <class K, bool ABI>
+// ABI: the C ABI's mode (arena in and out) or a batch's (outputs only). FAR: for launches with a plan of
+// more entries than 16 bits index (rare, and a kernel of its own, since the index's upper half costs
+// the others registers: df64 12 -> 24 bytes of spills, 65 537 points of the 3-jet mix 6.17 -> 6.29 ms)
+template <class K, bool ABI, bool FAR = false>
 __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
     typedef typename K::R R;
     typedef typename K::Den Den;
@@ -665,7 +679,7 @@ __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
         const uint32_t groups = 32 / np, x = threadIdx.x & 31, q = x / np, pw = x - q * np;
         const uint32_t tl = (threadIdx.x >> 5) * groups + q;
         const bool active = q < groups;
-        SlotView<K, ABI> v;
+        SlotView<K, ABI, 0, FAR> v;
         // forms, amplitudes, currents, terms, reciprocals: each region a multiple of the next one's
         // access size
         double *forms64 = (double *)(block + L.const_bytes);
@@ -734,9 +748,9 @@ __global__ void __launch_bounds__(512, 1) run_tiled(TiledLaunch L) {
             // plans at two blocks per SM) run a copy of the levels with that count built in; in the C
             // ABI's kernel more copies of the levels cost registers
             const bool all_near = p.near == p.entries;
-            if (!ABI && np == 1 && all_near)
+            if (!ABI && !FAR && np == 1 && all_near)
                 run_levels<K, ABI>(v.template with_points<1>(near), p, forms64, tl, active, plain);
-            else if (!ABI && np == 8 && all_near)
+            else if (!ABI && !FAR && np == 8 && all_near)
                 run_levels<K, ABI>(v.template with_points<8>(near), p, forms64, tl, active, plain);
             else
                 run_levels<K, ABI>(v, p, forms64, tl, active, plain);

@@ -12,7 +12,8 @@ struct KindF64Fma : Kind<double, double, double, double> {
     static constexpr bool contracted = true;
 };
 
-const void *tiled_fma_kernel(bool abi) {
+const void *tiled_fma_kernel(bool abi, bool far) {
+    if (far) return abi ? (const void *)run_tiled<KindF64Fma, true, true> : (const void *)run_tiled<KindF64Fma, false, true>;
     return abi ? (const void *)run_tiled<KindF64Fma, true> : (const void *)run_tiled<KindF64Fma, false>;
 }
 

@@ -52,7 +52,9 @@ struct Slab {
 }  // namespace
 
 // the f64 kind with contracted multiply-adds (tiled_fma.cu, compiled with -fmad=true)
-const void *tiled_fma_kernel(bool abi);
+const void *tiled_fma_kernel(bool abi, bool far);
+// the other kinds' kernels for tables of more entries than 16 bits index (tiled_far.cu)
+const void *tiled_far_kernel(int kernel, bool abi);
 void tiled_fma_fold(const uint32_t *entries, uint32_t count, const void *constants, uint32_t scales, uint32_t factors,
                     void *out, cudaStream_t s);
 
@@ -62,10 +64,11 @@ template <class K> const void *kernel_of(bool abi) {
     return abi ? (const void *)run_tiled<K, true> : (const void *)run_tiled<K, false>;
 }
 
-const void *kernel_for(int kernel, bool abi = false) {
+const void *kernel_for(int kernel, bool abi = false, bool far = false) {
+    if (far && kernel != PACUDA_B200_KERNEL_F64_FMA) return tiled_far_kernel(kernel, abi);
     switch (kernel) {
     case PACMAN_RECURRENCE_KERNEL_F64: return kernel_of<KindF64>(abi);
-    case PACUDA_B200_KERNEL_F64_FMA: return tiled_fma_kernel(abi);
+    case PACUDA_B200_KERNEL_F64_FMA: return tiled_fma_kernel(abi, far);
     case PACMAN_RECURRENCE_KERNEL_MIXED: return kernel_of<KindMixed>(abi);
     case PACMAN_RECURRENCE_KERNEL_MIXED64: return kernel_of<KindMixed64>(abi);
     default: return kernel_of<KindDF64>(abi);
@@ -85,9 +88,17 @@ void TiledDevice::release() {
 bool pack_ins(const Ins &i, bool end, uint4 &w) {
     // (a closure's f records its global amplitude plane for the host; the executor reads its slot)
     uint32_t f = ins_kind(i) == K_CLOSURE ? 0 : i.f, f0 = f & 0xffff, f1 = f >> 16;
-    if (ins_count(i) > C_GENERAL || f0 > 255 || f1 > 255 || i.a > 0xffff || i.b > 0xffff || i.c > 0xffff || i.s > 0xffff ||
-        i.x > 0xffff || i.y > 0xffff)
-        return false;
+    uint32_t a = i.a, b = i.b, c = i.c, s = i.s, x = i.x, y = i.y;
+    auto split = [](uint32_t &low, uint32_t &high) {  // an entry's index (Row16 entry_s, _x, _y)
+        high = low >> 16;
+        low &= 0xffff;
+    };
+    if (ins_kind(i) == K_CONTRIB && ins_op(i) != kOpLoad) split(s, x);
+    else if (ins_kind(i) == K_PROP || ins_kind(i) == K_IDENTITY) split(x, c);
+    else if (ins_kind(i) == K_CLOSURE) split(y, x);
+    for (uint32_t field : {a, b, c, s, x, y})
+        if (field > 0xffff) return false;
+    if (ins_count(i) > C_GENERAL || f0 > 255 || f1 > 255) return false;
     const uint32_t flags = ins_flags(i);
     const bool contribution = ins_kind(i) == K_CONTRIB && ins_op(i) != kOpLoad, last = !contribution || (flags & F_LAST);
     uint32_t head = row_code(i) | ins_count(i) << 4 | ins_op(i) << 8;
@@ -98,9 +109,9 @@ bool pack_ins(const Ins &i, bool end, uint4 &w) {
     if (contribution && (flags & F_FIRST) && (flags & F_INIT)) head |= H_SET;
     if (last && (flags & F_WB)) head |= H_WB;
     w.x = head | f0 << 16 | f1 << 24;
-    w.y = i.a | i.b << 16;
-    w.z = i.c | i.s << 16;
-    w.w = i.x | i.y << 16;
+    w.y = a | b << 16;
+    w.z = c | s << 16;
+    w.w = x | y << 16;
     return true;
 }
 
@@ -262,7 +273,7 @@ void describe(const TiledDevice &t, uint32_t forms, const PlanShape &shape, size
 }
 
 bool launch_tiled(int kernel, const TiledLaunch &args, int threads, size_t smem, int grid, cudaStream_t stream) {
-    const void *fn = kernel_for(kernel, args.abi);
+    const void *fn = kernel_for(kernel, args.abi, args.far);
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
     void *params[] = {(void *)&args};
     return cudaLaunchKernel(fn, dim3(grid), dim3(threads), params, smem, stream) == cudaSuccess;

@@ -55,6 +55,9 @@ struct TiledDevice {
 constexpr uint32_t kNearEntries = 256;
 inline size_t tiled_const_bytes(const TiledDevice &t) { return t.entry_count <= kNearEntries ? 16 * (size_t)t.entry_count : 0; }
 
+// whether a launch with the plan needs the kernels that read entries beyond 16 bits (tiled_far.cu)
+inline bool tiled_far(const TiledDevice &t) { return t.entry_count > 0x10000; }
+
 // a folded instruction (schedule.h Folds; `end`: its task's last) in the on-chip executor's 16-byte
 // form (tiled.cuh Row16); false when a field does not fit it
 bool pack_ins(const Ins &i, bool end, uint4 &w);
