@@ -784,11 +784,11 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs u) {
 // own issuing warp (one issues while the other waits), and the tiles' epilogues take turns, so that
 // one tile's activations run while the other's stores, barriers and products do; a warp loads its
 // accumulators before its turn. Sharing each chunk between two tiles halves the weights' L2 traffic.
-// Measured on B200, 2^21 points: 0.823 ms (109 cycles per point and SM, 1086 TFLOP/s, 0.65 of the
+// Measured on B200, 2^21 points: 0.83 ms (115 cycles per point and SM, 1077 TFLOP/s, 0.65 of the
 // measured BF16 peak); 0.846 with the accumulators loaded inside the turns, 0.903 without turns, 1.25
 // with one issuing warp for both tiles, 1.44 with that warp's loop on one lane (umma.cuh elect_one).
 // The form before (two blocks per SM, a tile each, a layer's products and its epilogue one after the
-// other): 1.31 ms. 300 007 points: 192 -> 126 us.
+// other): 1.31 ms. 300 007 points: 192 -> 131 us.
 // Each output's sums keep their order (k tiles 0 .. 3; the output layer's 128 columns of a half one
 // after the other): the bits do not depend on the split.
 

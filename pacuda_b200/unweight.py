@@ -164,7 +164,7 @@ class Pipeline:
         plans, moms, outs = self._parts([f.momenta[: 4 * f.legs * 1024] for f in self.fams], [1024] * nf)
         self.batch = B.Batch(plans, moms, outs)
         # until tune() has timed the plans' choices: by their points' size (a two-stage step of 2^22
-        # candidates, some 20 000 of them evaluated, 1.87 ms at one block per SM, 1.74 so)
+        # candidates: 1.80 ms at one block per SM, 1.71 so with 29 590 points evaluated, 2.61 and 2.33 with 51 224)
         self.batch.blocks_per_sm = 0
 
     def _parts(self, moms, counts):
