@@ -254,7 +254,7 @@ template <class K, bool ABI, int NP = 0, bool FAR = false> struct SlotView {
 // What bounds the executor is the instructions of a row (fetch, decode, moves, tests beside the
 // arithmetic) and their latency with 16 warps per SM, so the common rows each have a dispatch code
 // and straight code without class or flag tests: of gg>ggg's 22 900 warp instructions per point,
-// 12 600 of them FP64, 17 700 and 10 200 are left. Measured on B200, 4096 points of gg>ggg: 173 ->
+// 12 600 of them FP64, 17 200 and 10 150 are left. Measured on B200, 4096 points of gg>ggg: 173 ->
 // 146 us; 50 021 of qg>qgg with contracted multiply-adds: 430 -> 374 us; 65 537 of the 3-jet mix in
 // df64, where every product left out is about ten f32 instructions: 10.6 -> 6.95 ms. (The folded
 // constants alone, with class and flag tests in every row: no gain in f64.)

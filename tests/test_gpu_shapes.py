@@ -69,3 +69,28 @@ def test_blocks_per_sm_at_the_limit(blocks):
     b.run()
     torch.cuda.synchronize()
     same(out.cpu().numpy().reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("points,lanes", [(16, 32), (1, 512)])
+def test_the_runner_at_the_limit(points, lanes, tmp_path):
+    """The runner's on-chip executor at configured lanes per point (a process of its own: it is configured once)."""
+    import os
+    import subprocess
+    import sys
+
+    base = processes.template("qg>qgg")
+    forms = (ROOM // points - (16 * 632 + 16 * 96 + 32 * 15)) // 32  # its slots, amplitudes and forms in f64
+    code = f"""
+import numpy as np
+from pacuda_b200 import phase_space, processes, runner
+from tests.test_gpu_shapes import padded
+r = runner.Runner()
+assert r.configure("f64", executor="onchip", lanes_per_point={lanes}) == 0
+_, outs = r.evaluate(padded(processes.template("qg>qgg"), {forms}), phase_space.sample(5, 23, 4))
+np.save(r"{tmp_path / 'out.npy'}", outs)
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=600)
+    assert p.returncode == 0, p.stderr[-2000:]
+    _, want = O.evaluate(base, phase_space.sample(5, 23, 4), kernel=abi.KERNELS["f64"])
+    same(np.load(tmp_path / "out.npy").reshape(want.shape), want)
