@@ -530,6 +530,7 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
     // fewer leave more of a block's lanes idle at the levels' barriers) for each blocks-per-SM
     // choice, and the fastest pair; plans of the same blocks per SM share a launch
     const int kernel = b->plans[0]->kernel;
+    float alone = -1.0f;  // the last plan's best time
     for (size_t k = 0; k < b->plans.size(); k++) {
         pacuda_b200_plan *p = b->plans[k];
         float best = -1.0f;
@@ -551,6 +552,7 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
                 }
             }
         }
+        alone = best;
         if (best >= 0.0f) {
             p->size.points = best_points;
             p->size.chosen = true;
@@ -565,11 +567,14 @@ extern "C" int pacuda_b200_batch_tune(pacuda_b200_batch *b, void *stream) {
         b->exec = nullptr;
         b->graph = nullptr;
     }
-    // a batch of few points: all of it at its pairs and spread over the SMs, the best of three each
+    // A batch of few points: all of it at its pairs (one plan's is timed already) and spread over the SMs,
+    // the best of three each; nothing where the pairs are that launch.
+    bool same = true;
+    for (size_t k = 0; k < b->plans.size(); k++) same = same && b->plan_blocks[k] == 1 && b->plans[k]->size.points == 1;
     b->spread_counts = b->count;
-    if (few_points(b)) {
-        float ms[2] = {-1.0f, -1.0f};
-        for (int spread = 0; spread < 2; spread++) {
+    if (!same && few_points(b)) {
+        float ms[2] = {b->plans.size() == 1 ? alone : -1.0f, -1.0f};
+        for (int spread = b->plans.size() == 1; spread < 2; spread++) {
             b->spread_counts = spread ? b->count : std::vector<uint32_t>();
             bool ok = wait_copied(b) && prepare(b) && launch(b, s) == PACMAN_RECURRENCE_OK;
             for (int rep = 0; ok && rep < 3; rep++) {
